@@ -4,7 +4,7 @@
 // FP64 path (k_paint64): one thread per particle, the reference's double arithmetic,
 // global FP64 atomics into zeroed grids. It is the plain FP64 GPU path.
 //
-// FP32 path (k_bucket -> k_tile_rec -> k_edge_fixup; deterministic: k_count -> k_scan -> k_scatter ->
+// FP32 path (k_bucket_cta or k_bucket_warp -> k_tile_rec -> k_edge_fixup; deterministic: k_count -> k_scan -> k_scatter ->
 // k_tile_rec_det): particles are bucketed into the output tiles their stencils touch (a counting sort; a particle near a tile face is
 // listed in each neighbouring tile), then one CTA per tile accumulates every stencil tap of
 // its particles in shared memory and writes the tile once with coalesced stores. Every grid
@@ -15,6 +15,8 @@
 // the reference bit for bit. The deterministic variant accumulates int64 fixed point in shared memory.
 #include <cuda_runtime.h>
 #include <math.h>
+
+#include <algorithm>
 
 #include "paint.cuh"
 #include "paint_dev.cuh"
@@ -486,132 +488,435 @@ __global__ void __launch_bounds__(256) k_scatter(Geom g, FieldSpec fs, TileGeo t
   }
 }
 
-// Bucket mode, passes 1-3 in one: the statistics of k_count and the records of k_scatter, each
-// written into its tile's fixed-capacity bucket (slot from the run-aggregated tile counter); a
-// record that finds its bucket full goes to the overflow list with its tile. (Four CTAs per SM:
-// 64 registers, which the overlapped reservations below need without spilling.)
-template <typename T>
-__global__ void __launch_bounds__(256, 4) k_bucket(Geom g, FieldSpec fs, TileGeo tg, PIn<T> in, long long n,
-                                                   long long ibase, unsigned *counts, float4 *recs, float *recw, unsigned cap,
-                                                unsigned *edge_list, unsigned *edge_count, float4 *ovf_recs,
-                                                float *ovf_w, unsigned *ovf_tile, unsigned *ovf_count,
-                                                unsigned long long ovf_cap, DevStats *st) {
-  float f_read = 0, f_out = 0, f_nsq = 0, f_v[4] = {0, 0, 0, 0}, f_abs[2] = {0, 0}, f_grid = 0;
-  int fatal = 0, nonfin = 0, ovf_full = 0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
-    const long long i = i0 + (threadIdx.x & 31);
-    bool has = false;
-    AxisTiles TX, TY, TZ;
-    TX.n = TY.n = TZ.n = 0;
-    float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
-    float w = 1.0f;
-    if (i < n) {
-      const Prep p = prep32(g, fs, in, i);
-      if (!p.fin) {
-        nonfin = 1;
-      } else {
-        f_read += 1.0f;
-        if (fs.moments) {  // src/read_data.c:132-138, every particle read
-          f_nsq += p.w;
-          float wv = p.w * p.v;
-          f_v[0] += wv; wv *= p.v;
-          f_v[1] += wv; wv *= p.v;
-          f_v[2] += wv; wv *= p.v;
-          f_v[3] += wv;
-        }
-        float pa = p.w, pb = p.w;
-        for (int e = 0; e < fs.ea; e++) pa *= p.v;
-        for (int e = 0; e < fs.eb; e++) pb *= p.v;
-        f_abs[0] += fabsf(pa);
-        f_abs[1] += fabsf(pb);
-        if (!footprint(g, tg, p.sx, p.sy, p.sz, TX, TY, TZ)) {
-          f_out += 1.0f;  // clearly outside the box (src/read_data.c:81-88)
-          if (g.los == 0) {
-            fatal = 1;
-            atomicMax(&st->fatal_inv, ~0ULL - (unsigned long long)(ibase + i));
-          }
-        } else if (is_edge(g, p.sx, p.sy, p.sz)) {
-          edge_list[atomicAdd(edge_count, 1u)] = (unsigned)(ibase + i);  // painted and counted by k_edge_fixup
-        } else {
-          has = true;
-          w = p.w;
-          rec = make_float4(p.sx, p.sy, p.sz, p.v);
-          if (accept32(g, p.sx, p.sy, p.sz)) f_grid += p.w;  // NGRID (src/read_data.c:92-126)
-          if (outside32(g, p.sx, p.sy, p.sz)) f_out += 1.0f;  // src/read_data.c:81-88
-        }
-      }
-    }
-    const int na = __reduce_max_sync(FULL_MASK, has ? TX.n : 0), nb = __reduce_max_sync(FULL_MASK, has ? TY.n : 0),
-              nc = __reduce_max_sync(FULL_MASK, has ? TZ.n : 0);
-    auto put = [&](int key, unsigned slot) {
-      if (key < 0) return;
-      if (slot < cap) {
-        const unsigned long long r = (unsigned long long)key * cap + slot;
-        recs[r] = rec;
-        if (recw) recw[r] = w;
-      } else {
-        const unsigned o = atomicAdd(ovf_count, 1u);
-        if (o < ovf_cap) {
-          ovf_recs[o] = rec;
-          if (ovf_w) ovf_w[o] = w;
-          ovf_tile[o] = (unsigned)key;
-        } else {
-          ovf_full = 1;
-        }
-      }
-    };
-    if (na <= 2 && nb <= 2 && nc <= 2) {
-      // every (a, b, c) reservation of the warp first (their atomics in flight together), then the
-      // records: lane slot = the run head's returned base + the lane's place in its run
-      const int lane = threadIdx.x & 31;
-      int keys[8], hd[8];
-      unsigned base[8];
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const int a = t >> 2, b = (t >> 1) & 1, c = t & 1;
-        keys[t] = -1;
-        hd[t] = 0;
-        base[t] = 0;
-        if (a < na && b < nb && c < nc) {  // warp-uniform
-          const int key = tile_key(tg, has, TX, TY, TZ, a, b, c);
-          const int prev = __shfl_up_sync(FULL_MASK, key, 1);
-          const unsigned heads = __ballot_sync(FULL_MASK, lane == 0 || key != prev);
-          const unsigned after = heads & ~((2u << lane) - 1u);
-          const int head = 31 - __clz(heads & ((2u << lane) - 1u));
-          if (head == lane && key >= 0) base[t] = atomicAdd(counts + key, (unsigned)((after ? __ffs(after) - 1 : 32) - lane));
-          keys[t] = key;
-          hd[t] = head;
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const int a = t >> 2, b = (t >> 1) & 1, c = t & 1;
-        if (a < na && b < nb && c < nc) {
-          const unsigned b0 = __shfl_sync(FULL_MASK, base[t], hd[t]);
-          put(keys[t], b0 + (unsigned)(lane - hd[t]));
-        }
-      }
-    } else {
-      // runtime loops over the warp's footprint tiles (warp-uniform bounds): one copy of the body
-#pragma unroll 1
-      for (int a = 0; a < na; a++)
-#pragma unroll 1
-        for (int b = 0; b < nb; b++)
-#pragma unroll 1
-          for (int c = 0; c < nc; c++) {
-            const int key = tile_key(tg, has, TX, TY, TZ, a, b, c);
-            put(key, warp_run_add(counts, key, true));
-          }
-    }
+// The tiles of one particle as a first tile and per-axis extents: tile (a, b, c), a < nx, b < ny, c < nz, is
+// id + a SX + b SY + c SZ less a whole axis of tiles where a (b, c) has passed the axis's wrap (kx, ky, kz:
+// the first wrapped step). footprint()'s lists are consecutive tiles modulo the axis, so this holds them all.
+struct Foot {
+  unsigned id, ext;  // ext: nx, ny, nz, kx, ky, kz in 2 bits each
+};
+
+__device__ __forceinline__ Foot pack_foot(const TileGeo &tg, const AxisTiles &TX, const AxisTiles &TY,
+                                          const AxisTiles &TZ) {
+  Foot f;
+  f.id = (unsigned)tile_id(tg, TX.t0, TY.t0, TZ.t0);
+  const int kx = min(tg.nbx - TX.t0, 3), ky = min(tg.nby - TY.t0, 3), kz = min(tg.nbz - TZ.t0, 3);
+  f.ext = (unsigned)(TX.n | TY.n << 2 | TZ.n << 4 | kx << 6 | ky << 8 | kz << 10);
+  return f;
+}
+
+// Tile k < nx ny nz of a footprint (z fastest).
+__device__ __forceinline__ int foot_tile(const TileGeo &tg, const Foot &f, int k) {
+  const int nz = (f.ext >> 4) & 3, ny = (f.ext >> 2) & 3;
+  const int q = nz == 1 ? k : (nz == 2 ? k >> 1 : (k * 86) >> 8);  // k / nz for k < 27
+  const int c = k - q * nz;
+  const int a = ny == 1 ? q : (ny == 2 ? q >> 1 : (q * 86) >> 8);
+  const int b = q - a * ny;
+  int id = (int)f.id + (a * tg.nby + b) * tg.nbz + c;
+  if (a >= (int)((f.ext >> 6) & 3)) id -= tg.ntiles;
+  if (b >= (int)((f.ext >> 8) & 3)) id -= tg.nby * tg.nbz;
+  if (c >= (int)((f.ext >> 10) & 3)) id -= tg.nbz;
+  return id;
+}
+
+// A particle whose stencils lie inside the grid by whole cells along every axis: no edge of the reference's
+// rules within reach, accepted, inside the box, and its footprint neither wraps nor is clipped. (NN has an
+// edge at every cell, so it never qualifies.) s and s + 1/2 in [1 + m, n - 2 - m], m the margin.
+__device__ __forceinline__ bool interior32(const Geom &g, float sx, float sy, float sz) {
+  const float lo = 1.0f + 2.0f * g.margin, off = 2.5f + 2.0f * g.margin;
+  return (g.order > 1) & (sx >= lo) & (sx <= (float)g.nx - off) & (sy >= lo) & (sy <= (float)g.ny - off) & (sz >= lo) &
+         (sz <= (float)g.nz - off);
+}
+
+// axis_footprint of an interior particle: first tile and tile count (at most 3: six cells, tiles of four or more).
+__device__ __forceinline__ void axis_interior(float s, float m, int order, int shift, int &t0, int &n) {
+  const int lo = __float2int_rd(__fsub_rn(s, m)) - (order == 3 ? 1 : 0), hi = __float2int_rd(__fadd_rn(s, m)) + 2;
+  t0 = lo >> shift;
+  n = (hi >> shift) - t0 + 1;
+}
+
+// Compensated FP32 sum (the rounding error of each addition is carried to the next one): a thread of the
+// bucketing sums a hundred particles, and the mean velocity that the shot noise of a cross spectrum takes
+// from these sums is a small difference of large ones.
+struct CSum {
+  float s, c;
+  __device__ __forceinline__ CSum() : s(0.0f), c(0.0f) {}
+  __device__ __forceinline__ void add(float v) {
+    const float y = __fsub_rn(v, c), u = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(u, s), y);
+    s = u;
   }
-  const float vals[10] = {f_read, f_out, f_nsq, f_v[0], f_v[1], f_v[2], f_v[3], f_abs[0], f_abs[1], f_grid};
-  double *const dst[10] = {&st->nread, &st->nout, &st->nsq, &st->vr[0], &st->vr[1], &st->vr[2], &st->vr[3],
-                           &st->absw[0], &st->absw[1], &st->ngrid};
-  block_add_f<10>(vals, dst);
-  if (fatal) atomicOr(&st->fatal, 1);
-  if (nonfin) atomicOr(&st->nonfinite, 1);
-  if (ovf_full) atomicOr(&st->overflow, 1);
+};
+
+// Block sum of NV compensated sums, each warp's in pairs of floats (the pair's high part s and what its
+// additions rounded away), FP64 across warps, added to global dst.
+template <int NV>
+__device__ void block_add_cs(const CSum (&v)[NV], double *const (&dst)[NV]) {
+  __shared__ double redc[32][NV];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    float hi = v[k].s, lo = -v[k].c;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float h2 = __shfl_xor_sync(FULL_MASK, hi, o), l2 = __shfl_xor_sync(FULL_MASK, lo, o);
+      const float u = __fadd_rn(hi, h2), b = __fsub_rn(u, hi);
+      lo = __fadd_rn(__fadd_rn(lo, l2), __fadd_rn(__fsub_rn(hi, __fsub_rn(u, b)), __fsub_rn(h2, b)));
+      hi = u;
+    }
+    if (lane == 0) redc[wid][k] = (double)hi + (double)lo;
+  }
+  __syncthreads();
+  if (wid == 0 && lane < NV) {
+    double a = 0.0;
+    for (int w = 0; w < nw; w++) a += redc[w][lane];
+    if (a != 0.0) atomicAdd(dst[lane], a);
+  }
+  __syncthreads();
+}
+
+// One particle's sums (src/read_data.c:132-138 and the fixed-point bound), over a thread's particles.
+struct BucketSums {
+  float read, out, abs_a, abs_b;
+  CSum nsq, v[4], grid;
+  int fatal, nonfin;
+  __device__ __forceinline__ BucketSums() : read(0.0f), out(0.0f), abs_a(0.0f), abs_b(0.0f), fatal(0), nonfin(0) {}
+  __device__ __forceinline__ void add_read(const FieldSpec &fs, const Prep &q) {
+    read += 1.0f;
+    if (fs.moments) {  // every particle read
+      nsq.add(q.w);
+      float wv = q.w * q.v;
+      v[0].add(wv); wv *= q.v;
+      v[1].add(wv); wv *= q.v;
+      v[2].add(wv); wv *= q.v;
+      v[3].add(wv);
+    }
+    float pa = q.w, pb = q.w;
+    for (int e = 0; e < fs.ea; e++) pa *= q.v;
+    for (int e = 0; e < fs.eb; e++) pb *= q.v;
+    abs_a += fabsf(pa);
+    abs_b += fabsf(pb);
+  }
+  __device__ __forceinline__ void finish(DevStats *st, int ovf_full) {
+    const float vals[4] = {read, out, abs_a, abs_b};
+    double *const dst[4] = {&st->nread, &st->nout, &st->absw[0], &st->absw[1]};
+    block_add_f<4>(vals, dst);
+    const CSum cs[6] = {grid, nsq, v[0], v[1], v[2], v[3]};
+    double *const dc[6] = {&st->ngrid, &st->nsq, &st->vr[0], &st->vr[1], &st->vr[2], &st->vr[3]};
+    block_add_cs<6>(cs, dc);
+    if (fatal) atomicOr(&st->fatal, 1);
+    if (nonfin) atomicOr(&st->nonfinite, 1);
+    if (ovf_full) atomicOr(&st->overflow, 1);
+  }
+};
+
+constexpr unsigned FOOT_NONE = 0xffffffffu;  // a particle with no tiles: one empty entry
+
+// Footprint of an interior particle.
+__device__ __forceinline__ Foot interior_foot(const Geom &g, const TileGeo &tg, float sx, float sy, float sz) {
+  int tx, ty, tz, nx, ny, nz;
+  axis_interior(sx, g.margin, g.order, tg.lx, tx, nx);
+  axis_interior(sy, g.margin, g.order, tg.ly, ty, ny);
+  axis_interior(sz, g.margin, g.order, tg.lz, tz, nz);
+  Foot f;
+  f.id = (unsigned)tile_id(tg, tx, ty, tz);
+  f.ext = (unsigned)(nx | ny << 2 | nz << 4 | 0xfc0);
+  return f;
+}
+
+// Footprint of any other particle by the full rules (idx its catalogue index): none when it is outside or
+// goes to the exact rules.
+__device__ __forceinline__ Foot near_foot(const Geom &g, const TileGeo &tg, float sx, float sy, float sz, float w,
+                                          long long idx, unsigned *edge_list, unsigned *edge_count, DevStats *st,
+                                          BucketSums &sum) {
+  Foot f;
+  f.id = FOOT_NONE;
+  f.ext = 0x15;
+  AxisTiles TX, TY, TZ;
+  TX.n = TY.n = TZ.n = 0;
+  if (!footprint(g, tg, sx, sy, sz, TX, TY, TZ)) {
+    sum.out += 1.0f;  // clearly outside the box (src/read_data.c:81-88)
+    if (g.los == 0) {
+      sum.fatal = 1;
+      atomicMax(&st->fatal_inv, ~0ULL - (unsigned long long)idx);
+    }
+  } else if (is_edge(g, sx, sy, sz)) {
+    edge_list[atomicAdd(edge_count, 1u)] = (unsigned)idx;  // painted and counted by k_edge_fixup
+  } else {
+    f = pack_foot(tg, TX, TY, TZ);
+    if (accept32(g, sx, sy, sz)) sum.grid.add(w);        // NGRID (src/read_data.c:92-126)
+    if (outside32(g, sx, sy, sz)) sum.out += 1.0f;
+  }
+  return f;
+}
+
+// A warp's particles spread over its lanes: with cnt (at least 1) tiles of this lane's particle, entry e of the
+// warp belongs to the particle whose first entry is the last one at or before e. next() gives the owner of
+// entry t + lane for t = 0, 32, ...
+struct WarpSpread {
+  int off, total, before;
+  __device__ __forceinline__ WarpSpread(int cnt, int lane) {
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(FULL_MASK, incl, o);
+      if (lane >= o) incl += u;
+    }
+    off = incl - cnt;
+    total = __shfl_sync(FULL_MASK, incl, 31);
+    before = 0;
+  }
+  __device__ __forceinline__ int next(int t, int lane) {
+    const unsigned firsts = __reduce_or_sync(FULL_MASK, (unsigned)(off - t) < 32u ? 1u << (off - t) : 0u);
+    const int own = before + __popc(firsts & (0xffffffffu >> (31 - lane))) - 1;
+    before += __popc(firsts);
+    return own;
+  }
+};
+
+// Where records go: their tile's bucket, or when it is full the overflow list.
+struct BucketOut {
+  float4 *recs;
+  float *recw;
+  unsigned cap;
+  float4 *ovf_recs;
+  float *ovf_w;
+  unsigned *ovf_tile, *ovf_count;
+  unsigned long long ovf_cap;
+  __device__ __forceinline__ int put(int key, unsigned slot, const float4 &rec, float w) const {
+    if (slot < cap) {
+      const unsigned long long r = (unsigned long long)key * cap + slot;
+      recs[r] = rec;
+      if (recw) recw[r] = w;
+      return 0;
+    }
+    const unsigned o = atomicAdd(ovf_count, 1u);
+    if (o >= ovf_cap) return 1;
+    ovf_recs[o] = rec;
+    if (ovf_w) ovf_w[o] = w;
+    ovf_tile[o] = (unsigned)key;
+    return 0;
+  }
+};
+
+// One-pass bucketing, passes 1-3 in one: the statistics of k_count and the records of k_scatter, each written
+// into its tile's fixed-capacity bucket; a record that finds its bucket full goes to the overflow list with its
+// tile. A particle has 1.1 to 2.9 entries (tiles); a warp spreads its particles' entries over its lanes, so that
+// they cost no idle lanes, and lanes with equal tiles share one reservation of bucket slots. What bounds both
+// variants below is instruction issue. They differ in how slots are reserved.
+//
+// k_bucket_cta, for up to BK_DIRECT_TILES tiles: a CTA ranks the entries of a chunk of BK_THREADS * ppt
+// particles by shared counters of every tile, reserves each touched tile's slots with one global atomic, then
+// writes the records. With few tiles and particles in random order the global atomics of the warps would meet
+// on the same addresses: 2,097,152 such particles took 337 us into the 256 tiles of a 128^3 grid when each run
+// of lanes made its own.
+constexpr int BK_THREADS = 512;
+constexpr int BK_DIRECT_TILES = 4096;  // 16 KB of counters
+constexpr int BK_PPT = 4;              // particles per thread and chunk, at most
+constexpr int BK_P = BK_THREADS * BK_PPT;
+constexpr int BK_E = 4096;             // entries held; any beyond go out one by one
+
+static size_t bucket_smem(int ntiles) {
+  return sizeof(float4) * BK_P + 4 * BK_P + 4 * BK_E + 2 * BK_E + 2 * BK_P + 4 * (size_t)ntiles;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(BK_THREADS, 2)
+    k_bucket_cta(Geom g, FieldSpec fs, TileGeo tg, PIn<T> in, long long n, long long ibase, int ppt, unsigned *counts,
+                 BucketOut out, unsigned *edge_list, unsigned *edge_count, DevStats *st) {
+  extern __shared__ __align__(16) unsigned char smb[];
+  float4 *srec = (float4 *)smb;
+  float *sw = (float *)(srec + BK_P);
+  unsigned *shr = (unsigned *)(sw + BK_P);            // entry: tile | rank << 16
+  unsigned short *sown = (unsigned short *)(shr + BK_E);
+  unsigned short *slist = sown + BK_E;                // the chunk's particles near the grid's faces
+  unsigned *sc = (unsigned *)(slist + BK_P);          // counters, then the reserved first slots
+  __shared__ unsigned s_ent, s_near;
+  const int lane = threadIdx.x & 31;
+  for (int h = threadIdx.x; h < tg.ntiles; h += BK_THREADS) sc[h] = 0;
+  if (threadIdx.x == 0) s_ent = s_near = 0;
+  __syncthreads();
+  BucketSums sum;
+  int ovf_full = 0;
+  auto add_entries = [&](const Foot &ft, int li) {
+    WarpSpread ws((int)((ft.ext & 3) * ((ft.ext >> 2) & 3) * ((ft.ext >> 4) & 3)), lane);
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(&s_ent, (unsigned)ws.total);
+    base = __shfl_sync(FULL_MASK, base, 0);
+    for (int t = 0; t < ws.total; t += 32) {
+      const int own = ws.next(t, lane), e = t + lane;
+      Foot f;
+      f.id = __shfl_sync(FULL_MASK, ft.id, own);
+      f.ext = __shfl_sync(FULL_MASK, ft.ext, own);
+      const int k = e - __shfl_sync(FULL_MASK, ws.off, own), oli = __shfl_sync(FULL_MASK, li, own);
+      const unsigned pos = base + (unsigned)e;
+      const bool held = e < ws.total && pos < (unsigned)BK_E, real = e < ws.total && f.id != FOOT_NONE;
+      const int key = real ? foot_tile(tg, f, k) : -1;
+      // lanes of one tile take consecutive ranks from one counter access
+      const unsigned peers = __match_any_sync(FULL_MASK, held ? key : -1);
+      const int head = __ffs(peers) - 1;
+      unsigned rank = 0;
+      if (held && real && head == lane) rank = atomicAdd(&sc[key], (unsigned)__popc(peers));
+      rank = __shfl_sync(FULL_MASK, rank, head) + (unsigned)__popc(peers & ((1u << lane) - 1u));
+      if (held) {
+        shr[pos] = real ? (unsigned)key | rank << 16 : FOOT_NONE;
+        sown[pos] = (unsigned short)oli;
+      } else if (real) {  // more entries than the list holds (tiles that are small for the footprint)
+        ovf_full |= out.put(key, atomicAdd(counts + key, 1u), srec[oli], sw[oli]);
+      }
+    }
+  };
+  const int chunk = BK_THREADS * ppt;
+  for (long long c0 = (long long)blockIdx.x * chunk; c0 < n; c0 += (long long)gridDim.x * chunk) {
+#pragma unroll 1
+    for (int p = 0; p < ppt; p++) {
+      const int li = p * BK_THREADS + threadIdx.x;
+      const long long i = c0 + li;
+      if (i - lane >= n) break;  // the whole warp is past the end
+      Foot ft;
+      ft.id = FOOT_NONE;
+      ft.ext = 0x15;
+      if (i < n) {
+        const Prep q = prep32(g, fs, in, i);
+        if (!q.fin) {
+          sum.nonfin = 1;
+        } else {
+          sum.add_read(fs, q);
+          srec[li] = make_float4(q.sx, q.sy, q.sz, q.v);
+          sw[li] = q.w;
+          if (interior32(g, q.sx, q.sy, q.sz)) {
+            ft = interior_foot(g, tg, q.sx, q.sy, q.sz);
+            sum.grid.add(q.w);  // NGRID (src/read_data.c:92-126)
+          } else {
+            slist[atomicAdd(&s_near, 1u)] = (unsigned short)li;
+          }
+        }
+      }
+      __syncwarp();  // srec and sw of the warp's particles are written
+      add_entries(ft, li);
+    }
+    __syncthreads();
+    // the few particles near a face of the grid (for NN: all), by the full rules, in dense warps
+    const int nnear = (int)s_near;
+    for (int q0 = threadIdx.x - lane; q0 < nnear; q0 += BK_THREADS) {
+      const int q = q0 + lane, li = q < nnear ? slist[q] : 0;
+      Foot ft;
+      ft.id = FOOT_NONE;
+      ft.ext = 0x15;
+      if (q < nnear) {
+        const float4 r = srec[li];
+        ft = near_foot(g, tg, r.x, r.y, r.z, sw[li], ibase + c0 + li, edge_list, edge_count, st, sum);
+      }
+      add_entries(ft, li);
+    }
+    __syncthreads();
+    const int ne = (int)min(s_ent, (unsigned)BK_E);
+    for (int h = threadIdx.x; h < tg.ntiles; h += BK_THREADS) {
+      const unsigned c = sc[h];
+      if (c) sc[h] = atomicAdd(counts + h, c);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < ne; e += BK_THREADS) {
+      const unsigned hr = shr[e];
+      if (hr == FOOT_NONE) continue;
+      const int own = sown[e], key = (int)(hr & 0xffffu);
+      ovf_full |= out.put(key, sc[key] + (hr >> 16), srec[own], sw[own]);
+    }
+    __syncthreads();
+    for (int h = threadIdx.x; h < tg.ntiles; h += BK_THREADS) sc[h] = 0;
+    if (threadIdx.x == 0) s_ent = s_near = 0;
+    __syncthreads();
+  }
+  sum.finish(st, ovf_full);
+}
+
+// k_bucket_warp, for more tiles: the lanes of a warp with equal tiles share one global atomic, two groups of 32
+// entries at a time so that their atomics are in flight together, and the next particles' loads run behind
+// them. (A CTA-wide ranking through a hash table of the touched tiles was slower: 550 against 500 us for 16.7M
+// particles in lattice order at 512^3.)
+template <typename T>
+__global__ void __launch_bounds__(256, 4)
+    k_bucket_warp(Geom g, FieldSpec fs, TileGeo tg, PIn<T> in, long long n, long long ibase, unsigned *counts,
+                  BucketOut out, unsigned *edge_list, unsigned *edge_count, DevStats *st) {
+  __shared__ float4 s_rec[256];
+  __shared__ float s_w[256];
+  const int lane = threadIdx.x & 31;
+  float4 *wrec = s_rec + (threadIdx.x - lane);
+  float *ww = s_w + (threadIdx.x - lane);
+  BucketSums sum;
+  int ovf_full = 0;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x - lane; i0 < n; i0 += stride) {
+    const long long i = i0 + lane;
+    Foot ft;
+    ft.id = FOOT_NONE;
+    ft.ext = 0x15;
+    if (i < n) {
+      const Prep q = prep32(g, fs, in, i);
+      if (!q.fin) {
+        sum.nonfin = 1;
+      } else {
+        sum.add_read(fs, q);
+        wrec[lane] = make_float4(q.sx, q.sy, q.sz, q.v);
+        ww[lane] = q.w;
+        if (interior32(g, q.sx, q.sy, q.sz)) {
+          ft = interior_foot(g, tg, q.sx, q.sy, q.sz);
+          sum.grid.add(q.w);  // NGRID (src/read_data.c:92-126)
+        } else {
+          ft = near_foot(g, tg, q.sx, q.sy, q.sz, q.w, ibase + i, edge_list, edge_count, st, sum);
+        }
+      }
+    }
+    __syncwarp();
+    WarpSpread ws((int)((ft.ext & 3) * ((ft.ext >> 2) & 3) * ((ft.ext >> 4) & 3)), lane);
+    for (int t = 0; t < ws.total; t += 64) {
+      int key[2], own[2], head[2];
+      unsigned base[2], rank[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int e = t + 32 * u + lane;
+        own[u] = ws.next(t + 32 * u, lane) & 31;
+        Foot f;
+        f.id = __shfl_sync(FULL_MASK, ft.id, own[u]);
+        f.ext = __shfl_sync(FULL_MASK, ft.ext, own[u]);
+        const int k = e - __shfl_sync(FULL_MASK, ws.off, own[u]);
+        key[u] = e < ws.total && f.id != FOOT_NONE ? foot_tile(tg, f, k) : -1;
+        const unsigned peers = __match_any_sync(FULL_MASK, key[u]);
+        head[u] = __ffs(peers) - 1;
+        rank[u] = (unsigned)__popc(peers & ((1u << lane) - 1u));
+        base[u] = 0;
+        if (head[u] == lane && key[u] >= 0) base[u] = atomicAdd(counts + key[u], (unsigned)__popc(peers));
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const unsigned slot = __shfl_sync(FULL_MASK, base[u], head[u]) + rank[u];
+        if (key[u] >= 0) ovf_full |= out.put(key[u], slot, wrec[own[u]], ww[own[u]]);
+      }
+    }
+    __syncwarp();  // the next particles overwrite wrec
+  }
+  sum.finish(st, ovf_full);
+}
+
+template <typename T>
+static void launch_bucket(cudaStream_t s, const Geom &g, const FieldSpec &fs, const TileGeo &tg, const PIn<T> &in,
+                          long long n, long long ibase, const PaintBufs &b, DevStats *st) {
+  const BucketOut out{b.recs,     in.w ? b.recw : nullptr, b.bucket_cap, b.ovf_recs, in.w ? b.ovf_w : nullptr,
+                      b.ovf_tile, b.ovf_count,             b.ovf_cap};
+  if (tg.ntiles <= BK_DIRECT_TILES) {
+    const size_t smem = bucket_smem(tg.ntiles);
+    cudaFuncSetAttribute(k_bucket_cta<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one resident wave (two CTAs per SM); a small catalogue takes fewer particles per chunk, to fill it
+    const long long wave = 152LL * 2 * BK_THREADS;
+    const int ppt = (int)std::min<long long>(BK_PPT, std::max<long long>(1, n / wave));
+    const long long chunks = (n + BK_THREADS * ppt - 1) / (BK_THREADS * ppt);
+    const int nb = (int)(chunks < 1 ? 1 : (chunks > 152 * 2 ? 152 * 2 : chunks));
+    k_bucket_cta<T><<<nb, BK_THREADS, smem, s>>>(g, fs, tg, in, n, ibase, ppt, b.counts, out, b.edge_list, b.edge_count,
+                                                 st);
+  } else {
+    const long long nb = (n + 255) / 256;
+    k_bucket_warp<T><<<(int)(nb < 1 ? 1 : (nb > 152 * 8 ? 152 * 8 : nb)), 256, 0, s>>>(
+        g, fs, tg, in, n, ibase, b.counts, out, b.edge_list, b.edge_count, st);
+  }
 }
 
 // Deterministic accumulation: round(value * 2^S) added as an integer (S from k_scan, per field).
@@ -819,7 +1124,7 @@ __device__ __forceinline__ void tile_rec_deposit(const Geom &g, const FieldSpec 
 // deposit below 2^22, where rint_small rounds it). Lane = record: each thread reads one record, derives its taps
 // once per stencil and adds the K^3 products, so a record is read once and nothing is staged. The
 // cells are converted back to FP32 when the tile is written. (NGRID of these particles is counted
-// by k_bucket or k_count.)
+// by the bucketing or k_count.)
 template <int K, int NF, bool IL>
 __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileGeo tg, const unsigned *offsets,
                                                      const unsigned *counts, unsigned cap, const float4 *recs,
@@ -1489,11 +1794,7 @@ static void run_paint32(cudaStream_t s, const Geom &g, const FieldSpec &fs, cons
       const long long c0 = n * k / nch, c1 = n * (k + 1) / nch;
       if (nch > 1) cudaStreamWaitEvent(s, b.chunk_ev[k], 0);
       PIn<T> ink{in.x + c0, in.y + c0, in.z + c0, in.v ? in.v + c0 : nullptr, in.w ? in.w + c0 : nullptr};
-      const long long nbk = (c1 - c0 + th - 1) / th;
-      const int nbc = (int)(nbk < 1 ? 1 : (nbk > 152 * 8 ? 152 * 8 : nbk));
-      k_bucket<T><<<nbc, th, 0, s>>>(g, fs, tg, ink, c1 - c0, c0, b.counts, b.recs, in.w ? b.recw : nullptr,
-                                     b.bucket_cap, b.edge_list, b.edge_count, b.ovf_recs, in.w ? b.ovf_w : nullptr,
-                                     b.ovf_tile, b.ovf_count, b.ovf_cap, st);
+      launch_bucket<T>(s, g, fs, tg, ink, c1 - c0, c0, b, st);
     }
     *launches += nch - 1;
     const bool wts = in.w != nullptr;

@@ -212,7 +212,7 @@ extern "C" int capow_create(const capow_params *p, const capow_options *opt, cap
   CK(c, cudaMallocHost((void **)&c->h_bins, sizeof(double) * NPROD * (5 * nk + n2d)));
   CK(c, cudaMallocHost((void **)&c->h_st, sizeof(DevStats)));
   if (!f64) {
-    c->tg = choose_tiles(c->g, c->nslot, c->prec == CAPOW_FP32_DETERMINISTIC);
+    c->tg = c->prec == CAPOW_FP32_DETERMINISTIC ? choose_tiles(c->g, c->nslot, 1) : fit_tiles(c->g, c->nslot);
     c->pb.counts = (unsigned *)dalloc(c, sizeof(unsigned) * c->tg.ntiles);
     c->pb.offsets = (unsigned *)dalloc(c, sizeof(unsigned) * (c->tg.ntiles + 1));
     c->pb.cursor = (unsigned *)dalloc(c, sizeof(unsigned) * c->tg.ntiles);
@@ -365,7 +365,7 @@ int create_paint_ctx(const capow_params *p, const capow_options *o, int survey, 
     FAIL(c, CAPOW_ENOMEM, "device allocation failed (grids need %.2f GB)", eb * c->grid_elems * c->nslot / 1e9);
   CK(c, cudaMallocHost((void **)&c->h_st, sizeof(DevStats)));
   if (c->prec != CAPOW_FP64) {
-    c->tg = choose_tiles(c->g, c->nslot, c->prec == CAPOW_FP32_DETERMINISTIC);
+    c->tg = c->prec == CAPOW_FP32_DETERMINISTIC ? choose_tiles(c->g, c->nslot, 1) : fit_tiles(c->g, c->nslot);
     c->pb.counts = (unsigned *)dalloc(c, sizeof(unsigned) * c->tg.ntiles);
     c->pb.offsets = (unsigned *)dalloc(c, sizeof(unsigned) * (c->tg.ntiles + 1));
     c->pb.cursor = (unsigned *)dalloc(c, sizeof(unsigned) * c->tg.ntiles);

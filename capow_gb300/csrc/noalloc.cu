@@ -134,10 +134,12 @@ extern "C" int capow_paint_noalloc(capow_ctx *c, const capow_particles *parts) {
     }
   }
   const bool det = c->prec == CAPOW_FP32_DETERMINISTIC, weights = parts->w != nullptr;
-  const unsigned long long n = parts->n, per = records_per_particle(c->g, c->tg);
+  // the default tiles: a context's smaller ones on a small grid may list a particle more often
+  const TileGeo tg = choose_tiles(c->g, c->nslot, det ? 1 : 0);
+  const unsigned long long n = parts->n, per = records_per_particle(c->g, tg);
   const unsigned long long limit = CAPOW_NOALLOC_SCRATCH_BYTES;
   // size check before anything touches the device: the record count n * per must fit
-  const NoallocLayout fixed = noalloc_layout(c->tg, 0, 0, !det, weights);
+  const NoallocLayout fixed = noalloc_layout(tg, 0, 0, !det, weights);
   const unsigned long long per_bytes = per * (16ULL + (weights ? 4ULL : 0ULL)) + (det ? 0ULL : 4ULL);
   const unsigned long long fit = fixed.total + 1024 < limit ? (limit - fixed.total - 1024) / per_bytes : 0;
   if (n > fit || n * per >= 0xFFFFFFF0ULL)
@@ -145,7 +147,7 @@ extern "C" int capow_paint_noalloc(capow_ctx *c, const capow_particles *parts) {
          "capow_paint_noalloc: %llu particles exceed the fixed %llu-byte scratch (up to %llu tile records per "
          "particle on this grid); at most %llu particles fit",
          n, limit, per, fit);
-  const NoallocLayout L = noalloc_layout(c->tg, n, n * per, !det, weights);
+  const NoallocLayout L = noalloc_layout(tg, n, n * per, !det, weights);
   if (L.total > limit) FAIL(c, CAPOW_EINVAL, "capow_paint_noalloc: scratch layout exceeds the fixed array");
   CK(c, cudaSetDevice(c->o.device));
   void *base = nullptr;
@@ -178,7 +180,7 @@ extern "C" int capow_paint_noalloc(capow_ctx *c, const capow_particles *parts) {
     gp.g[k] = k < c->nslot ? (void *)((float *)c->grid_base + c->grid_elems * k) : nullptr;
   CK(c, cudaMemsetAsync(c->st, 0, sizeof(DevStats), c->stream));
   CK(c, cudaEventRecord(c->ev[0], c->stream));
-  launch_paint32(c->stream, c->g, c->fs, c->tg, det ? 1 : 0, d.dtype, d.x, d.y, d.z, d.vlos, d.w, (long long)n, gp,
+  launch_paint32(c->stream, c->g, c->fs, tg, det ? 1 : 0, d.dtype, d.x, d.y, d.z, d.vlos, d.w, (long long)n, gp,
                  b, c->st, &c->launches);
   CK(c, cudaGetLastError());
   CK(c, cudaEventRecord(c->ev[1], c->stream));

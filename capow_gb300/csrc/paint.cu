@@ -989,80 +989,20 @@ __device__ __forceinline__ int rint_small(float a, float b) {
 
 // The int32 quantum of a tile is about 2^-30 of the tile's total |w v^e|, and a cell sums up to one
 // rounded deposit per record: the cells' relative error grows with the record count. A tile with
-// more records than this (a dense clump; uniform catalogues put about a thousand records in a
-// tile) is accumulated in int64 with 2^61 headroom instead, one grid slot and one shared-memory
-// chunk of cells per pass over its records (the records are re-read from L2 for each pass).
-#define TILE_PRECISE_RECORDS 16384
+// more records than this (a dense clump or a coarse grid; ordinary catalogues put about a thousand records
+// in a tile) is accumulated in two int32 limbs per cell instead (tile_paint_dense). For a tile smaller than
+// the default one the limit goes down with its cells, so that it stands for the same density.
+#define TILE_DENSE_RECORDS 16384u
 
-template <int K, int NF, bool IL>
-__device__ void tile_paint_precise(const Geom &g, const FieldSpec &fs, const TileGeo &tg, const float4 *recs,
-                                   const float *recw, unsigned long long rb, unsigned long long re, float ta, float tb,
-                                   int x0, int y0, int z0, int ex, int ey, int ez, int pyz, int tsz,
-                                   long long *sm64, int chunk, GridPtrs grids, DevStats *st) {
-  constexpr int NS = IL ? 2 : 1;
-  const int S64a = 60 - ilogbf(fmaxf(ta * 1.001f, 1e-30f)), S64b = 60 - ilogbf(fmaxf(tb * 1.001f, 1e-30f));
-  for (int slot = 0; slot < NS * NF; slot++) {
-    const int sten = slot / NF, fld = slot % NF;
-    const int S64 = fld == 0 ? S64a : S64b;
-    const float sc = ldexpf(1.0f, S64 > 100 ? 100 : S64);
-    float dsum = 0.0f;
-    for (int c0 = 0; c0 < tsz; c0 += chunk) {
-      const int c1 = min(tsz, c0 + chunk);
-      for (int c = threadIdx.x; c < c1 - c0; c += blockDim.x) sm64[c] = 0;
-      __syncthreads();
-      for (unsigned long long r = rb + threadIdx.x; r < re; r += blockDim.x) {
-        const float4 rec = recs[r];
-        const float w = recw ? recw[r] : 1.0f;
-        float v = w;
-        const int e_n = fld == 0 ? fs.ea : fs.eb;
-        for (int e = 0; e < e_n; e++) v *= rec.w;
-        v *= sc;
-        const float sx = sten ? __fadd_rn(rec.x, 0.5f) : rec.x, sy = sten ? __fadd_rn(rec.y, 0.5f) : rec.y,
-                    sz = sten ? __fadd_rn(rec.z, 0.5f) : rec.z;
-        if (!accept32(g, sx, sy, sz)) continue;
-        AxisTapsF ax, ay, az;
-        axis32k<K>(sx, 0, g.nx, g.los, ax);
-        axis32k<K>(sy, 1, g.ny, g.los, ay);
-        axis32k<K>(sz, 1, g.nz, g.los, az);
-        float wx[3], wy[3], wz[3];
-        int ox[3], oy[3], oz[3];
-        stage_axis32(ax, x0, ex, pyz, wx, ox);
-        stage_axis32(ay, y0, ey, tg.tz, wy, oy);
-        stage_axis32(az, z0, ez, 1, wz, oz);
-#pragma unroll
-        for (int a = 0; a < K; a++)
-#pragma unroll
-          for (int b2 = 0; b2 < K; b2++) {
-            const float wxy = wx[a] * wy[b2];
-            const float pv = v * wxy;
-            const int oxy = ox[a] + oy[b2];
-#pragma unroll
-            for (int c = 0; c < K; c++) {
-              const int off = oxy + oz[c] - c0;
-              if (wxy != 0.0f && wz[c] != 0.0f && off >= 0 && off < c1 - c0)
-                atomicAdd((unsigned long long *)(sm64 + off), (unsigned long long)__float2ll_rn(pv * wz[c]));
-            }
-          }
-      }
-      __syncthreads();
-      const double inv = ldexp(1.0, -(S64 > 100 ? 100 : S64));
-      float *gp = (float *)grids.g[slot];
-      for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        const int rz = c & (tg.tz - 1), ly = (c >> tg.lz) & (tg.ty - 1), lx = c >> (tg.lz + tg.ly);
-        if (lx >= ex || ly >= ey || rz >= ez) continue;
-        const float val = (float)((double)sm64[c - c0] * inv);
-        gp[(long long)(x0 + lx) * g.slice + (long long)(y0 + ly) * g.row + z0 + rz] = val;
-        dsum += val;
-      }
-      __syncthreads();
-    }
-    const double vals[1] = {(double)dsum};
-    double *const dst1[1] = {&st->dc[slot]};
-    block_add<1>(vals, dst1);
-  }
+// Scaled values w v^e of a record's two fields.
+__device__ __forceinline__ void record_values(const FieldSpec &fs, const float4 &rec, float w, float &va, float &vb) {
+  va = w;
+  vb = w;
+  for (int e = 0; e < fs.ea; e++) va *= rec.w;
+  for (int e = 0; e < fs.eb; e++) vb *= rec.w;
 }
 
-// The deposits of a tile's records (lane = record; both stencils) into the int32 shared tile.
+// The deposits of the records [rb, re) into the int32 shared tile (lane = record; both stencils).
 // FASTR: rounded by rint_small (every deposit below 2^22); otherwise by conversion.
 template <int K, int NF, bool IL, bool FASTR>
 __device__ __forceinline__ void tile_rec_deposit(const Geom &g, const FieldSpec &fs, const TileGeo &tg,
@@ -1073,10 +1013,8 @@ __device__ __forceinline__ void tile_rec_deposit(const Geom &g, const FieldSpec 
   const int slotw = tg.slot;
   for (unsigned long long r = rb + threadIdx.x; r < re; r += blockDim.x) {
     const float4 rec = recs[r];
-    const float w = recw ? recw[r] : 1.0f;
-    float va = w, vb = w;
-    for (int e = 0; e < fs.ea; e++) va *= rec.w;
-    for (int e = 0; e < fs.eb; e++) vb *= rec.w;
+    float va, vb;
+    record_values(fs, rec, recw ? recw[r] : 1.0f, va, vb);
     va *= scA;
     vb *= scB;
 #pragma unroll
@@ -1116,33 +1054,212 @@ __device__ __forceinline__ void tile_rec_deposit(const Geom &g, const FieldSpec 
   }
 }
 
+// A deposit p (an FP32 value already in the tile's fixed point) split as p = h 2^k + l with
+// h = floor(p 2^-k) and l = p - h 2^k in [0, 2^k] (k <= 22, |h| < 2^22), both made integers by the FMA rounding
+// of rint_small and added with two native int32 shared atomics; the cell's value is hi 2^k + lo. The FMA
+// that forms l is exact except for a negative p of magnitude below 2^k, where the deposit may come out
+// one unit of the fixed point away from round(p): still a fixed function of p, whatever the order.
+__device__ __forceinline__ void limb_add(int *lo, int *hi, float p, float two_mk, float two_k) {
+  const float h = floorf(p * two_mk);
+  const float l = __fmaf_rn(-h, two_k, p);
+  atomicAdd(lo, rint_small(l, 1.0f));
+  atomicAdd(hi, rint_small(h, 1.0f));
+}
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The shared::cluster address of this CTA's shared address in CTA `rank` of the cluster, and loads from it.
+__device__ __forceinline__ unsigned map_cluster(unsigned smem, int rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ int ld_cluster_s32(unsigned a) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster_f32(unsigned a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// Place of a tile and of a CTA in the tile's cluster (of S CTAs, this one's rank).
+struct TileAt {
+  int x0, y0, z0, ex, ey, ez, S, rank;
+};
+
+// A tile's write-out: pairs of cells along z as float2 (8-byte aligned global rows). A thread keeps one (y, z)
+// pair of the tile's x-planes and walks x: the pair's address in shared memory and in the grid only advance by
+// px and the grid slice. cell(word) gives the pair at a shared word of a plane's slot; store(x, a0, a1) gets it.
+// In a cluster each CTA writes its share of the pairs and planes.
+template <bool CL, typename F>
+__device__ __forceinline__ void tile_walk(const Geom &g, const TileGeo &tg, const TileAt &at, F &&store) {
+  const int ppl = (tg.ty * tg.tz) >> 1;  // pairs per x-plane
+  const int nthr = (int)blockDim.x * at.S;
+  // a cluster has more threads than a plane has pairs: they share the x-planes
+  const int xs = CL ? max(1, min(at.ex, nthr / ppl)) : 1;
+  for (int q = at.rank * (int)blockDim.x + threadIdx.x; q < ppl * xs; q += nthr) {
+    const int w = CL ? q % ppl : q, lx0 = CL ? q / ppl : 0;
+    const int c = w << 1;
+    const int rz = c & (tg.tz - 1), ly = c >> tg.lz;
+    if (ly >= at.ey || rz >= at.ez) continue;
+    const bool two = rz + 1 < at.ez;
+    const int cb = ly * tg.py + rz;
+    const long long gb = (long long)at.x0 * g.slice + (long long)(at.y0 + ly) * g.row + at.z0 + rz;
+    for (int lx = lx0; lx < at.ex; lx += xs) store(cb + lx * tg.px, gb + (long long)lx * g.slice, two);
+  }
+}
+
+__device__ __forceinline__ float store_pair(float *dst, float a0, float a1, bool two) {
+  if (two) {
+    *reinterpret_cast<float2 *>(dst) = make_float2(a0, a1);
+    return a0 + a1;
+  }
+  dst[0] = a0;
+  return a0;
+}
+
+// A dense tile, one slot at a time: the records [r0, r1) of this CTA into cells of two int32 limbs (hi 2^17 + lo)
+// at a scale with (record count) (largest |w v^e|) 2^S < 2^47, which leaves a deposit its FP32 product for any
+// count; every 8192 records the low limbs' carries go to the high ones. Two native atomics a deposit: before
+// (int64 cells with 64-bit shared atomics, in chunks of a slot) 5.4M weighted particles took 32 ms into a 32^3
+// grid, 16.7M into 256^3 1.28 ms.
+constexpr int DENSE_K = 17;
+constexpr unsigned DENSE_ROUND = 8192;
+
+template <int K, int NF, bool IL, bool CL>
+__device__ void tile_paint_dense(const Geom &g, const FieldSpec &fs, const TileGeo &tg, const float4 *recs,
+                                 const float *recw, unsigned long long r0, unsigned long long r1, float xa, float xb,
+                                 const TileAt &at, int *smi, float *s_inv, GridPtrs grids, DevStats *st) {
+  constexpr int NS = IL ? 2 : 1;
+  const int slotw = tg.slot;
+  int *lo = smi, *hi = smi + slotw;
+  const float cnt = (float)(r1 - r0);
+  const float bound[2] = {cnt * xa * 1.001f, cnt * xb * 1.001f};
+  int Sx[2];
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const int S = bound[f] > 0.0f && isfinite(bound[f]) ? 46 - ilogbf(bound[f]) : 0;
+    Sx[f] = S > 100 ? 100 : (S < -100 ? -100 : S);
+  }
+  if (threadIdx.x == 0) {
+    s_inv[0] = ldexpf(1.0f, -Sx[0]);
+    s_inv[1] = ldexpf(1.0f, -Sx[1]);
+  }
+  const float two_k = (float)(1 << DENSE_K), two_mk = 1.0f / two_k;
+#pragma unroll 1
+  for (int slot = 0; slot < NS * NF; slot++) {
+    const int sten = slot / NF, fld = slot % NF;
+    const float sc = ldexpf(1.0f, fld ? Sx[1] : Sx[0]);
+    for (int c = threadIdx.x; c < 2 * slotw; c += blockDim.x) smi[c] = 0;
+    __syncthreads();
+    for (unsigned long long rr = r0; rr < r1; rr += DENSE_ROUND) {
+      if (rr > r0) {  // carries of the records so far
+        __syncthreads();
+        for (int c = threadIdx.x; c < slotw; c += blockDim.x) {
+          const int v = lo[c];
+          hi[c] += v >> DENSE_K;
+          lo[c] = v & ((1 << DENSE_K) - 1);
+        }
+        __syncthreads();
+      }
+      const unsigned long long rt = min(r1, rr + DENSE_ROUND);
+      for (unsigned long long r = rr + threadIdx.x; r < rt; r += blockDim.x) {
+        const float4 rec = recs[r];
+        float va, vb;
+        record_values(fs, rec, recw ? recw[r] : 1.0f, va, vb);
+        const float v = (fld ? vb : va) * sc;
+        const float sx = sten ? __fadd_rn(rec.x, 0.5f) : rec.x, sy = sten ? __fadd_rn(rec.y, 0.5f) : rec.y,
+                    sz = sten ? __fadd_rn(rec.z, 0.5f) : rec.z;
+        if (!accept32(g, sx, sy, sz)) continue;
+        AxisTapsF ax, ay, az;
+        axis32k<K>(sx, 0, g.nx, g.los, ax);
+        axis32k<K>(sy, 1, g.ny, g.los, ay);
+        axis32k<K>(sz, 1, g.nz, g.los, az);
+        float wx[3], wy[3], wz[3];
+        int ox[3], oy[3], oz[3];
+        stage_axis32(ax, at.x0, at.ex, tg.px, wx, ox);
+        stage_axis32(ay, at.y0, at.ey, tg.py, wy, oy);
+        stage_axis32(az, at.z0, at.ez, 1, wz, oz);
+#pragma unroll
+        for (int a = 0; a < K; a++)
+#pragma unroll
+          for (int b2 = 0; b2 < K; b2++) {
+            const float wxy = wx[a] * wy[b2];
+            if (wxy == 0.0f) continue;
+            const float pv = v * wxy;
+            const int oxy = ox[a] + oy[b2];
+#pragma unroll
+            for (int c = 0; c < K; c++)
+              if (wz[c] != 0.0f) limb_add(lo + oxy + oz[c], hi + oxy + oz[c], pv * wz[c], two_mk, two_k);
+          }
+      }
+    }
+    if (CL) cluster_sync_all();
+    else __syncthreads();
+    float *gp = (float *)grids.g[slot];
+    float dsum = 0.0f;
+    const unsigned la = (unsigned)__cvta_generic_to_shared(lo), ha = (unsigned)__cvta_generic_to_shared(hi),
+                   ia = (unsigned)__cvta_generic_to_shared(s_inv + fld);
+    tile_walk<CL>(g, tg, at, [&](int cp, long long go, bool two) {
+      float a0 = 0.0f, a1 = 0.0f;
+      if (CL) {
+        for (int k = 0; k < at.S; k++) {
+          const unsigned l = map_cluster(la, k) + 4 * cp, h = map_cluster(ha, k) + 4 * cp;
+          const float inv = ld_cluster_f32(map_cluster(ia, k));
+          a0 += (float)(((long long)ld_cluster_s32(h) << DENSE_K) + ld_cluster_s32(l)) * inv;
+          a1 += (float)(((long long)ld_cluster_s32(h + 4) << DENSE_K) + ld_cluster_s32(l + 4)) * inv;
+        }
+      } else {
+        const float inv = ldexpf(1.0f, -(fld ? Sx[1] : Sx[0]));
+        a0 = (float)(((long long)hi[cp] << DENSE_K) + lo[cp]) * inv;
+        a1 = (float)(((long long)hi[cp + 1] << DENSE_K) + lo[cp + 1]) * inv;
+      }
+      dsum += store_pair(gp + go, a0, a1, two);
+    });
+    const float vals[1] = {dsum};
+    double *const dst1[1] = {&st->dc[slot]};
+    block_add_f<1>(vals, dst1);
+    if (CL) cluster_sync_all();  // every CTA has read this one's cells
+  }
+}
+
 // FP32 tile kernel for particles away from every edge of the reference's rules (those are painted
-// by k_edge_fixup). One CTA per tile; shared memory holds the tile of every grid slot, both
-// stencils, [tx][ty][tz] with the padded pitches py = 3, px = 9 (mod 32) so that deposits at equal z
-// spread over the banks, as int32 fixed point with a per-tile power-of-two scale, so
-// every deposit is one native integer shared-memory atomic (an ordinary tile's scale also keeps each
-// deposit below 2^22, where rint_small rounds it). Lane = record: each thread reads one record, derives its taps
-// once per stencil and adds the K^3 products, so a record is read once and nothing is staged. The
-// cells are converted back to FP32 when the tile is written. (NGRID of these particles is counted
-// by the bucketing or k_count.)
-template <int K, int NF, bool IL>
+// by k_edge_fixup). One CTA per tile, or (CL) a cluster of `split` CTAs that share a tile's records; shared
+// memory holds the tile of every grid slot, both stencils, [tx][ty][tz] with the padded pitches py = 3, px = 9
+// (mod 32) so that deposits at equal z spread over the banks, as int32 fixed point with a per-CTA
+// power-of-two scale, so every deposit is one native integer shared-memory atomic (an ordinary tile's scale
+// also keeps each deposit below 2^22, where rint_small rounds it). Lane = record: each thread reads one
+// record, derives its taps once per stencil and adds the K^3 products, so a record is read once and nothing
+// is staged. The cells are converted back to FP32 when the tile is written; in a cluster each CTA writes its
+// share of the tile as the sum of every CTA's cells (through distributed shared memory). (NGRID of these
+// particles is counted by the bucketing or k_count.)
+template <int K, int NF, bool IL, bool CL>
 __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileGeo tg, const unsigned *offsets,
                                                      const unsigned *counts, unsigned cap, const float4 *recs,
-                                                     const float *recw, unsigned long long capacity, GridPtrs grids,
-                                                     DevStats *st) {
+                                                     const float *recw, unsigned long long capacity, int split,
+                                                     unsigned dense, GridPtrs grids, DevStats *st) {
   extern __shared__ __align__(16) int smi[];
-  constexpr int NS = IL ? 2 : 1;
-  const int tsz = tg.tx * tg.ty * tg.tz;
-  const int pyz = tg.ty * tg.tz;
-  const int tile = blockIdx.x;
+  constexpr int NS = IL ? 2 : 1, SL = NS * NF;
+  TileAt at;
+  at.S = CL ? split : 1;
+  const int tile = CL ? blockIdx.x / at.S : blockIdx.x;
+  at.rank = CL ? blockIdx.x - tile * at.S : 0;
   const int bz = tile % tg.nbz, by = (tile / tg.nbz) % tg.nby, bx = tile / (tg.nbz * tg.nby);
-  const int x0 = bx * tg.tx, y0 = by * tg.ty, z0 = bz * tg.tz;
-  const int ex = min(tg.tx, g.nx - x0), ey = min(tg.ty, g.ny - y0), ez = min(tg.tz, g.nz - z0);
+  at.x0 = bx * tg.tx;
+  at.y0 = by * tg.ty;
+  at.z0 = bz * tg.tz;
+  at.ex = min(tg.tx, g.nx - at.x0);
+  at.ey = min(tg.ty, g.ny - at.y0);
+  at.ez = min(tg.tz, g.nz - at.z0);
   int4 *sm4 = reinterpret_cast<int4 *>(smi);
   const int slotw = tg.slot;  // words per padded slot
-  for (int c = threadIdx.x; c < (NS * NF * slotw) >> 2; c += blockDim.x) sm4[c] = make_int4(0, 0, 0, 0);
-  for (int c = ((NS * NF * slotw) & ~3) + threadIdx.x; c < NS * NF * slotw; c += blockDim.x) smi[c] = 0;
-  __syncthreads();
+  for (int c = threadIdx.x; c < (SL * slotw) >> 2; c += blockDim.x) sm4[c] = make_int4(0, 0, 0, 0);
+  for (int c = ((SL * slotw) & ~3) + threadIdx.x; c < SL * slotw; c += blockDim.x) smi[c] = 0;
   unsigned long long rb, re;
   if (cap) {  // bucket mode: the tile's own bucket
     rb = (unsigned long long)tile * cap;
@@ -1153,16 +1270,20 @@ __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileG
   }
   if (re > capacity) re = capacity;
   if (rb > re) rb = re;
-  // pre-pass over the tile's records: sum |w v^e| per field (the records stay in L1 for the deposits)
-  __shared__ float red_abs[4][32];
+  const unsigned cnt = (unsigned)(re - rb);
+  if (CL) {  // this CTA's share
+    const unsigned per = (cnt + (unsigned)at.S - 1) / (unsigned)at.S;
+    rb = min(re, rb + (unsigned long long)at.rank * per);
+    re = min(re, rb + per);
+  }
+  // pre-pass over the records: sum and largest |w v^e| per field (the records stay in L1 for the deposits)
+  __shared__ float red_abs[4][8];
+  __shared__ float s_inv[2];  // 1 / scale of the CTA's cells per field
   {
     float la = 0.0f, lb = 0.0f, ma = 0.0f, mb = 0.0f;
     for (unsigned long long r = rb + threadIdx.x; r < re; r += blockDim.x) {
-      const float4 rec = recs[r];
-      const float w = recw ? recw[r] : 1.0f;
-      float va = w, vb = w;
-      for (int e = 0; e < fs.ea; e++) va *= rec.w;
-      for (int e = 0; e < fs.eb; e++) vb *= rec.w;
+      float va, vb;
+      record_values(fs, recs[r], recw ? recw[r] : 1.0f, va, vb);
       la += fabsf(va);
       lb += fabsf(vb);
       ma = fmaxf(ma, fabsf(va));
@@ -1190,7 +1311,11 @@ __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileG
     xa = fmaxf(xa, red_abs[2][k]);
     xb = fmaxf(xb, red_abs[3][k]);
   }
-  // The tile's scale is set by its sum (tile_scale_exp). When keeping every deposit below 2^22 costs
+  if (cnt > dense) {  // uniform over the tile's CTAs
+    tile_paint_dense<K, NF, IL, CL>(g, fs, tg, recs, recw, rb, re, xa, xb, at, smi, s_inv, grids, st);
+    return;
+  }
+  // The scale is set by the sum (tile_scale_exp). When keeping every deposit below 2^22 costs
   // it at most 2 bits (an ordinary tile: hundreds of comparable records), the tile takes that scale
   // and the fast rounding; otherwise (few records, or one dominant record) it keeps the sum's scale
   // and rounds by conversion.
@@ -1198,74 +1323,55 @@ __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileG
   const int SAf = min(SAs, tile_scale_max(xa)), SBf = min(SBs, tile_scale_max(xb));
   const bool fast = (SAs - SAf <= 2) && (NF == 1 || SBs - SBf <= 2);
   const int SA = fast ? SAf : SAs, SB = fast ? SBf : SBs;
-  if (re - rb > TILE_PRECISE_RECORDS) {  // a dense tile (uniform over the CTA)
-    const int words = NS * NF * tsz;  // the int32 tile area, reused as int64 cells
-    tile_paint_precise<K, NF, IL>(g, fs, tg, recs, recw, rb, re, ta, tb, x0, y0, z0, ex, ey, ez, pyz, tsz,
-                                  reinterpret_cast<long long *>(smi), words / 2, grids, st);
-    return;
-  }
   const float scA = ldexpf(1.0f, SA), scB = ldexpf(1.0f, SB);
-  if (fast) tile_rec_deposit<K, NF, IL, true>(g, fs, tg, recs, recw, rb, re, scA, scB, x0, y0, z0, ex, ey, ez, smi);
-  else tile_rec_deposit<K, NF, IL, false>(g, fs, tg, recs, recw, rb, re, scA, scB, x0, y0, z0, ex, ey, ez, smi);
-  __syncthreads();
-  // write every slot: pairs of cells along z as float2 (8-byte aligned global rows). A thread keeps
-  // one (y, z) pair of the tile's x-planes and walks x, all slots per step: the pair's address in
-  // shared memory and in the grid only advance by px and the grid slice. The slots' DC sums go to
-  // one block reduction at the end (FP32 per thread and warp, FP64 across warps).
-  float dsums[NS * NF], invs[NS * NF];
+  if (CL && threadIdx.x == 0) {
+    s_inv[0] = ldexpf(1.0f, -SA);
+    s_inv[1] = ldexpf(1.0f, -SB);
+  }
+  if (fast) tile_rec_deposit<K, NF, IL, true>(g, fs, tg, recs, recw, rb, re, scA, scB, at.x0, at.y0, at.z0, at.ex, at.ey, at.ez, smi);
+  else tile_rec_deposit<K, NF, IL, false>(g, fs, tg, recs, recw, rb, re, scA, scB, at.x0, at.y0, at.z0, at.ex, at.ey, at.ez, smi);
+  if (CL) cluster_sync_all();
+  else __syncthreads();
+  // write every slot. The slots' DC sums go to one block reduction at the end (FP32 per thread and warp,
+  // FP64 across warps).
+  float dsums[SL], invs[SL];
 #pragma unroll
-  for (int slot = 0; slot < NS * NF; slot++) {
+  for (int slot = 0; slot < SL; slot++) {
     dsums[slot] = 0.0f;
     invs[slot] = ldexpf(1.0f, -((slot % NF) == 0 ? SA : SB));
   }
-  const int ppl = (tg.ty * tg.tz) >> 1;  // pairs per x-plane
-  for (int w = threadIdx.x; w < ppl; w += blockDim.x) {
-    const int c = w << 1;
-    const int rz = c & (tg.tz - 1), ly = c >> tg.lz;
-    if (ly >= ey || rz >= ez) continue;
-    const bool two = rz + 1 < ez;
-    const int cb = ly * tg.py + rz;
-    const long long gb = (long long)x0 * g.slice + (long long)(y0 + ly) * g.row + z0 + rz;
-    for (int lx = 0; lx < ex; lx++) {
-      const int cp = cb + lx * tg.px;
-      const long long go = gb + (long long)lx * g.slice;
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smi), ia = (unsigned)__cvta_generic_to_shared(s_inv);
+  tile_walk<CL>(g, tg, at, [&](int cp, long long go, bool two) {
 #pragma unroll
-      for (int slot = 0; slot < NS * NF; slot++) {
-        const int *sl = smi + slot * slotw + cp;
-        const float a0 = (float)sl[0] * invs[slot], a1 = (float)sl[1] * invs[slot];
-        float *dst = (float *)grids.g[slot] + go;
-        if (two) {
-          dsums[slot] += a0 + a1;
-          *reinterpret_cast<float2 *>(dst) = make_float2(a0, a1);
-        } else {
-          dsums[slot] += a0;
-          dst[0] = a0;
+    for (int slot = 0; slot < SL; slot++) {
+      float a0, a1;
+      if (CL) {
+        a0 = a1 = 0.0f;
+        for (int k = 0; k < at.S; k++) {
+          const unsigned q = map_cluster(sa, k) + 4 * (slot * slotw + cp);
+          const float inv = ld_cluster_f32(map_cluster(ia, k) + 4 * (slot % NF));
+          a0 += (float)ld_cluster_s32(q) * inv;
+          a1 += (float)ld_cluster_s32(q + 4) * inv;
         }
+      } else {
+        const int *sl = smi + slot * slotw + cp;
+        a0 = (float)sl[0] * invs[slot];
+        a1 = (float)sl[1] * invs[slot];
       }
+      dsums[slot] += store_pair((float *)grids.g[slot] + go, a0, a1, two);
     }
-  }
-  double *dsts[NS * NF];
+  });
+  double *dsts[SL];
 #pragma unroll
-  for (int slot = 0; slot < NS * NF; slot++) dsts[slot] = &st->dc[slot];
-  block_add_f<NS * NF>(dsums, dsts);
+  for (int slot = 0; slot < SL; slot++) dsts[slot] = &st->dc[slot];
+  block_add_f<SL>(dsums, dsts);
+  if (CL) cluster_sync_all();  // every CTA has read this one's cells
 }
 
 // --------------------------------------------------------------------- deterministic tile paint
 // Tiles with at most this many records accumulate in two-limb cells at a tile scale; denser ones in
 // uint64 cells at the run's global scale (64-bit shared atomics: slower, and rare).
 #define DET_FAST_RECORDS 8192u
-
-// A deposit p (an FP32 value already in the tile's fixed point, |p| < 2^40) split as p = h 2^k + l with
-// h = floor(p 2^-k) and l = p - h 2^k in [0, 2^k] (k <= 22), both made integers by the FMA rounding of
-// rint_small and added with two native int32 shared atomics; the cell's value is hi 2^k + lo. The FMA
-// that forms l is exact except for a negative p of magnitude below 2^k, where the deposit may come out
-// one unit of the fixed point away from round(p): still a fixed function of p, whatever the order.
-__device__ __forceinline__ void limb_add(int *lo, int *hi, float p, float two_mk, float two_k) {
-  const float h = floorf(p * two_mk);
-  const float l = __fmaf_rn(-h, two_k, p);
-  atomicAdd(lo, rint_small(l, 1.0f));
-  atomicAdd(hi, rint_small(h, 1.0f));
-}
 
 // Scale exponent of a tile: (record count) * (largest |w v^e| of its records) * 2^S < 2^40, so that no
 // cell of one pass (each record adds at most |w v^e| 2^S to a cell) leaves the limbs' range. Both inputs
@@ -1694,6 +1800,15 @@ TileGeo choose_tiles(const Geom &g, int nslots, int deterministic) {
   return make_tiles(g, nslots <= 2 ? 16 : 8, 16, 32);
 }
 
+// The FP32 tiles of a context: the default ones, or for a small grid smaller ones, so that there is about one
+// tile for each SM (rec_split then adds CTAs). (Edges below 8 would put a footprint in three tiles along an axis.)
+TileGeo fit_tiles(const Geom &g, int nslots) {
+  static const int edge[5][3] = {{16, 16, 32}, {16, 16, 16}, {8, 16, 16}, {8, 8, 16}, {8, 8, 8}};
+  TileGeo t = choose_tiles(g, nslots, 0);
+  for (int k = nslots <= 2 ? 1 : 2; k < 5 && t.ntiles < 152; k++) t = make_tiles(g, edge[k][0], edge[k][1], edge[k][2]);
+  return t;
+}
+
 // Tile edges are powers of two (tile coordinates are shifts); a grid edge shorter than the tile
 // uses the next power of two and the tile is partial.
 TileGeo make_tiles(const Geom &g, int tx, int ty, int tz) {
@@ -1723,7 +1838,8 @@ size_t tile_smem_bytes(const TileGeo &tg, int nslots, int deterministic) {
   return ((size_t)nslots * tg.slot * (deterministic ? 8 : 4) + 15) & ~(size_t)15;
 }
 
-size_t rec_smem_bytes(const TileGeo &tg, int nslots) { return (size_t)nslots * tg.slot * 4; }
+// k_tile_rec's cells: every slot, or for a dense tile the two limbs of one slot.
+size_t rec_smem_bytes(const TileGeo &tg, int nslots) { return (size_t)(nslots < 2 ? 2 : nslots) * tg.slot * 4; }
 
 double tile_dup_estimate(const Geom &g, const TileGeo &tg) {
   // a footprint spans 4 (TSC, CIC) or 2 (NN) cells plus the margin; it crosses into the next tile
@@ -1732,13 +1848,44 @@ double tile_dup_estimate(const Geom &g, const TileGeo &tg) {
   return (1.0 + (span - 1.0) / tg.tx) * (1.0 + (span - 1.0) / tg.ty) * (1.0 + (span - 1.0) / tg.tz);
 }
 
+// CTAs per tile (a cluster, a power of two up to 8): a grid of few tiles takes clusters that fill the chip (three
+// CTAs per SM), but no more CTAs than there are blocks of 128 records in a tile.
+static int rec_split(const TileGeo &tg, double records) {
+  int s = 1;
+  while (s < 8 && 2 * s * tg.ntiles <= 152 * 3 * 2 && records / tg.ntiles >= 128.0 * 2 * s) s *= 2;
+  return s;
+}
+
 template <int K, int NF, bool IL>
 static void launch_rec(cudaStream_t s, const Geom &g, const FieldSpec &fs, const TileGeo &tg, const PaintBufs &b,
-                       bool weights, const GridPtrs &grids, DevStats *st) {
+                       bool weights, long long n, const GridPtrs &grids, DevStats *st) {
   const size_t smem = rec_smem_bytes(tg, NF * (IL ? 2 : 1));
-  cudaFuncSetAttribute(k_tile_rec<K, NF, IL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_tile_rec<K, NF, IL><<<tg.ntiles, 256, smem, s>>>(g, fs, tg, b.offsets, b.counts, b.bucket_cap, b.recs,
-                                                     weights ? b.recw : nullptr, b.capacity, grids, st);
+  const int split = rec_split(tg, tile_dup_estimate(g, tg) * (double)n);
+  const float *recw = weights ? b.recw : nullptr;
+  const TileGeo def = choose_tiles(g, NF * (IL ? 2 : 1), 0);
+  const unsigned dense = (unsigned)((double)TILE_DENSE_RECORDS * std::min(1.0, (double)tg.tx * tg.ty * tg.tz /
+                                                                               ((double)def.tx * def.ty * def.tz)));
+  if (split > 1) {
+    cudaFuncSetAttribute(k_tile_rec<K, NF, IL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)split;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tg.ntiles * split));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_tile_rec<K, NF, IL, true>, g, fs, tg, (const unsigned *)b.offsets,
+                       (const unsigned *)b.counts, b.bucket_cap, (const float4 *)b.recs, recw, b.capacity, split, dense,
+                       grids, st);
+  } else {
+    cudaFuncSetAttribute(k_tile_rec<K, NF, IL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_tile_rec<K, NF, IL, false><<<tg.ntiles, 256, smem, s>>>(g, fs, tg, b.offsets, b.counts, b.bucket_cap, b.recs,
+                                                                   recw, b.capacity, 1, dense, grids, st);
+  }
   if (b.bucket_cap)
     k_ovf_paint<K, NF, IL><<<152 * 2, 128, 0, s>>>(g, fs, tg, b.ovf_recs, weights ? b.ovf_w : nullptr, b.ovf_tile,
                                                    b.ovf_count, b.ovf_cap, grids, st);
@@ -1746,13 +1893,13 @@ static void launch_rec(cudaStream_t s, const Geom &g, const FieldSpec &fs, const
 
 template <int K>
 static void launch_rec_k(cudaStream_t s, const Geom &g, const FieldSpec &fs, const TileGeo &tg, const PaintBufs &b,
-                         bool weights, const GridPtrs &grids, DevStats *st) {
+                         bool weights, long long n, const GridPtrs &grids, DevStats *st) {
   if (fs.nfields == 2) {
-    if (g.interlace) launch_rec<K, 2, true>(s, g, fs, tg, b, weights, grids, st);
-    else launch_rec<K, 2, false>(s, g, fs, tg, b, weights, grids, st);
+    if (g.interlace) launch_rec<K, 2, true>(s, g, fs, tg, b, weights, n, grids, st);
+    else launch_rec<K, 2, false>(s, g, fs, tg, b, weights, n, grids, st);
   } else {
-    if (g.interlace) launch_rec<K, 1, true>(s, g, fs, tg, b, weights, grids, st);
-    else launch_rec<K, 1, false>(s, g, fs, tg, b, weights, grids, st);
+    if (g.interlace) launch_rec<K, 1, true>(s, g, fs, tg, b, weights, n, grids, st);
+    else launch_rec<K, 1, false>(s, g, fs, tg, b, weights, n, grids, st);
   }
 }
 
@@ -1799,9 +1946,9 @@ static void run_paint32(cudaStream_t s, const Geom &g, const FieldSpec &fs, cons
     *launches += nch - 1;
     const bool wts = in.w != nullptr;
     if (b.tile_ev0) cudaEventRecord(b.tile_ev0, s);
-    if (g.order == 3) launch_rec_k<3>(s, g, fs, tg, b, wts, grids, st);
-    else if (g.order == 2) launch_rec_k<2>(s, g, fs, tg, b, wts, grids, st);
-    else launch_rec_k<1>(s, g, fs, tg, b, wts, grids, st);
+    if (g.order == 3) launch_rec_k<3>(s, g, fs, tg, b, wts, n, grids, st);
+    else if (g.order == 2) launch_rec_k<2>(s, g, fs, tg, b, wts, n, grids, st);
+    else launch_rec_k<1>(s, g, fs, tg, b, wts, n, grids, st);
     if (b.tile_ev1) cudaEventRecord(b.tile_ev1, s);
     k_edge_fixup<T><<<152 * 2, 128, 0, s>>>(g, fs, in, b.edge_list, b.edge_count, grids, st);
     *launches += 4;
@@ -1821,9 +1968,9 @@ static void run_paint32(cudaStream_t s, const Geom &g, const FieldSpec &fs, cons
   } else {
     const bool wts = in.w != nullptr;
     if (b.tile_ev0) cudaEventRecord(b.tile_ev0, s);
-    if (g.order == 3) launch_rec_k<3>(s, g, fs, tg, b, wts, grids, st);
-    else if (g.order == 2) launch_rec_k<2>(s, g, fs, tg, b, wts, grids, st);
-    else launch_rec_k<1>(s, g, fs, tg, b, wts, grids, st);
+    if (g.order == 3) launch_rec_k<3>(s, g, fs, tg, b, wts, n, grids, st);
+    else if (g.order == 2) launch_rec_k<2>(s, g, fs, tg, b, wts, n, grids, st);
+    else launch_rec_k<1>(s, g, fs, tg, b, wts, n, grids, st);
     if (b.tile_ev1) cudaEventRecord(b.tile_ev1, s);
     k_edge_fixup<T><<<152 * 2, 128, 0, s>>>(g, fs, in, b.edge_list, b.edge_count, grids, st);
     *launches += 5;

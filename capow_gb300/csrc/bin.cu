@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "bin.cuh"
+#include "fft_dev.cuh"
 #include "harm.cuh"
 #include "paint.cuh"
 
@@ -623,13 +624,6 @@ CAPOW_HD XbinSmem xbin_smem_layout(int log2n, int ncol, int np, int nl, int nk, 
   return L;
 }
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cmul_mi(float2 a) { return make_float2(a.y, -a.x); }  // a * (-i)
-
 // A column element read once: no L1 allocation, and an L2 fetch of the surrounding 256 bytes (the
 // neighbouring kz blocks of the same row, which other CTAs read next).
 __device__ __forceinline__ float2 ld_col(const float2 *p) {
@@ -638,37 +632,8 @@ __device__ __forceinline__ float2 ld_col(const float2 *p) {
   return v;
 }
 
-// In-place DIF butterflies of one stage, forward sign. Inputs a[q] at span/R spacing; outputs X[p]
-// (p in natural order) times the twiddle w^(p*j) are written back at position p.
-__device__ __forceinline__ void dft8(float2 *a) {
-  const float h = 0.70710678118654752f;
-  float2 b0 = cadd(a[0], a[4]), b4 = csub(a[0], a[4]);
-  float2 b1 = cadd(a[1], a[5]), t5 = csub(a[1], a[5]);
-  float2 b2 = cadd(a[2], a[6]), t6 = csub(a[2], a[6]);
-  float2 b3 = cadd(a[3], a[7]), t7 = csub(a[3], a[7]);
-  const float2 b5 = make_float2((t5.x + t5.y) * h, (t5.y - t5.x) * h);    // * e^{-i pi/4}
-  const float2 b6 = cmul_mi(t6);                                           // * e^{-i pi/2}
-  const float2 b7 = make_float2((t7.y - t7.x) * h, -(t7.x + t7.y) * h);   // * e^{-3i pi/4}
-  const float2 c0 = cadd(b0, b2), c2 = csub(b0, b2), c1 = cadd(b1, b3), c3 = cmul_mi(csub(b1, b3));
-  const float2 c4 = cadd(b4, b6), c6 = csub(b4, b6), c5 = cadd(b5, b7), c7 = cmul_mi(csub(b5, b7));
-  a[0] = cadd(c0, c1);
-  a[4] = csub(c0, c1);
-  a[2] = cadd(c2, c3);
-  a[6] = csub(c2, c3);
-  a[1] = cadd(c4, c5);
-  a[5] = csub(c4, c5);
-  a[3] = cadd(c6, c7);
-  a[7] = csub(c6, c7);
-}
-
-__device__ __forceinline__ void dft4(float2 *a) {
-  const float2 b0 = cadd(a[0], a[2]), b2 = csub(a[0], a[2]), b1 = cadd(a[1], a[3]), b3 = cmul_mi(csub(a[1], a[3]));
-  a[0] = cadd(b0, b1);
-  a[2] = csub(b0, b1);
-  a[1] = cadd(b2, b3);
-  a[3] = csub(b2, b3);
-}
-
+// In-place DIF butterflies of one stage take inputs a[q] at span/R spacing; outputs X[p] (p in natural order)
+// times the twiddle w^(p*j) are written back at position p.
 // a[p] *= w[p], p = 1..7, w one 16-byte aligned row of a stage's twiddle table (w[0] = 1)
 __device__ __forceinline__ void twiddle8(float2 *a, const float2 *w) {
   const float4 *w4 = (const float4 *)w;
@@ -1067,55 +1032,23 @@ __device__ ZrTables zr2c_load_tables(const BinTables &t, int log2m, unsigned cha
   return z;
 }
 
-// The z pass's loads: a pair of consecutive reals of row y of plane x (z = 2n, 2n + 1), read once. A load
-// functor's row(x, y) gives what is fixed along one row, and its load(p, n) reads pair n at p.
-struct ZrPlainRow {
-  __device__ __forceinline__ float2 load(const float2 *p, int) const { return __ldcs(p); }
-};
-struct ZrPlainLoad {
-  __device__ __forceinline__ ZrPlainRow row(int, int) const { return ZrPlainRow(); }
-};
-
 // One block of the z pass: ZB rows y0.. of plane x of slot sl, through the shared data area sd
 // ([M][ZB + 1]). The caller has synchronised after the tables were written and after any earlier use
-// of sd. ld reads the input pairs (ZrPlainLoad, or a weighting load). SP = 2: the block holds ZB / 2
-// rows of each of the slots sl and sl + 1 (columns r and r + ZB / 2 are row y0 + r of each), and one
-// thread reads the same cells of both, so that a weighting load's weights are evaluated once for both.
-template <int ZB, class LD = ZrPlainLoad, int SP = 1>
+// of sd. (The one-launch z + y transform's form for rows of 512 or more complex values.)
+template <int ZB>
 __device__ __forceinline__ void zr2c_block(const ZrGeo &zg, const ZrTables &z, const float *in, float2 *out,
-                                           float2 *sd, int sl, int x, int y0, const LD &ld = LD()) {
+                                           float2 *sd, int sl, int x, int y0) {
   constexpr int LZB = ZB == 16 ? 4 : 3;
-  constexpr int RS = ZB / SP;  // rows of each slot
   const int log2m = zg.log2m, M = 1 << log2m, P = ZB + 1, Q1 = M >> 3;
   const float *src = in + sl * zg.in_slot + (long long)x * zg.slice;
   // first DIF stage (span M) straight from the rows: butterfly (row r, jj) reads z[jj + q M/8];
   // lanes run along a row, so each of a warp's 8 loads is one contiguous 256-byte piece
-  for (int u = threadIdx.x; u < (RS << (log2m - 3)); u += blockDim.x) {
+  for (int u = threadIdx.x; u < (ZB << (log2m - 3)); u += blockDim.x) {
     const int jj = u & (Q1 - 1), r = u >> (log2m - 3), y = y0 + r;
     const float2 *rp = reinterpret_cast<const float2 *>(src + (long long)(y < zg.ny ? y : 0) * zg.row) + jj;
-    const auto rw = ld.row(x, y < zg.ny ? y : 0);  // what the row's loads share (a weighting load's row terms)
     float2 a[8];
-    if constexpr (SP == 1) {
 #pragma unroll
-      for (int q = 0; q < 8; q++) a[q] = y < zg.ny ? rw.load(rp + q * Q1, jj + q * Q1) : make_float2(0.0f, 0.0f);
-    } else {
-      const float2 *rpb = rp + (zg.in_slot >> 1);  // the same row of slot sl + 1 (in_slot floats is even)
-      float2 b[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        a[q] = b[q] = make_float2(0.0f, 0.0f);
-        if (y < zg.ny) {
-          const float2 w = rw.weights(jj + q * Q1), va = __ldcs(rp + q * Q1), vb = __ldcs(rpb + q * Q1);
-          a[q] = make_float2(va.x * w.x, va.y * w.y);
-          b[q] = make_float2(vb.x * w.x, vb.y * w.y);
-        }
-      }
-      dft8(b);
-      if (jj > 0) twiddle8(b, z.stw + 8 * jj);
-      float2 *pb = sd + jj * P + r + RS;
-#pragma unroll
-      for (int q = 0; q < 8; q++) pb[q * Q1 * P] = b[q];
-    }
+    for (int q = 0; q < 8; q++) a[q] = y < zg.ny ? __ldcs(rp + q * Q1) : make_float2(0.0f, 0.0f);
     dft8(a);
     if (jj > 0) twiddle8(a, z.stw + 8 * jj);
     float2 *p = sd + jj * P + r;
@@ -1164,9 +1097,9 @@ __device__ __forceinline__ void zr2c_block(const ZrGeo &zg, const ZrTables &z, c
   // real-input split and transposed store, X[k] and X[M-k] from the same pair: with
   // A = Z[k] + conj Z[M-k], B = Z[k] - conj Z[M-k] and w^M = -1, X[k] = (A + (-i) w^k B) / 2 and
   // X[M-k] = (conj A + (-i) conj(w^k B)) / 2. The thread's column r is the same on every step.
-  const int r = threadIdx.x & (ZB - 1), y = y0 + r % RS, so = r / RS;
+  const int r = threadIdx.x & (ZB - 1), y = y0 + r;
   if (y < zg.ny) {
-    float2 *dst = out + (sl + so) * zg.out_slot + (long long)x * zg.nzc * zg.ny + y;
+    float2 *dst = out + sl * zg.out_slot + (long long)x * zg.nzc * zg.ny + y;
     for (int k = threadIdx.x >> LZB; k <= (M >> 1); k += blockDim.x >> LZB) {
       const float2 zk = sd[z.spos[k & (M - 1)] * P + r];
       const float2 zm = sd[z.spos[(M - k) & (M - 1)] * P + r];
@@ -1179,30 +1112,6 @@ __device__ __forceinline__ void zr2c_block(const ZrGeo &zg, const ZrTables &z, c
   }
 }
 
-template <int ZB>
-__global__ void __launch_bounds__(ZR_THREADS) k_zr2c(ZrGeo zg, BinTables t, const float *in, float2 *out) {
-  extern __shared__ __align__(16) unsigned char smz[];
-  const int M = 1 << zg.log2m;
-  float2 *sd = (float2 *)smz;  // [M][ZB + 1]
-  const ZrTables z = zr2c_load_tables(t, zg.log2m, smz + align16(8u * (unsigned)M * (ZB + 1)));
-  const int per_slot = zg.nx * zg.nyb, nblk = per_slot * zg.ns;
-  for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {  // (slot, x, block of ZB rows)
-    const int sl = blk / per_slot, rem = blk - sl * per_slot;
-    const int x = rem / zg.nyb, y0 = (rem - x * zg.nyb) * ZB;
-    __syncthreads();  // tables written; the previous block's output has read sd
-    // the CTA's next block is ZB contiguous padded rows: one bulk prefetch into L2 while this one runs
-    const int nb = blk + (int)gridDim.x;
-    if (threadIdx.x == 0 && nb < nblk) {
-      const int sl2 = nb / per_slot, rem2 = nb - sl2 * per_slot;
-      const int x2 = rem2 / zg.nyb, y2 = (rem2 - x2 * zg.nyb) * ZB;
-      const float *nxt = in + sl2 * zg.in_slot + (long long)x2 * zg.slice + (long long)y2 * zg.row;
-      const unsigned bytes = ((unsigned)(min(ZB, zg.ny - y2) * zg.row) * 4u) & ~15u;
-      if (bytes && (((unsigned long long)nxt & 15ull) == 0))
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(nxt), "r"(bytes) : "memory");
-    }
-    zr2c_block<ZB>(zg, z, in, out, sd, sl, x, y0);
-  }
-}
 
 // The survey estimator's weighted z pass: the input of a set (l, m) is the painted grid times h_lm(r^) of
 // each cell (harm.cuh), applied as the rows are read, so that no weighted grid is written.
@@ -1211,99 +1120,174 @@ struct ZrWeight {
   int l, m;
 };
 
-// One row (plane x, row y) of a set: its harmonic's polynomial in pz (HarmRow, formed once per row), so
-// that a cell's weight is a Horner step per degree, one rsqrt and L - 1 products.
-template <int L>
-struct ZrWeightRow {
-  HarmRow<L> h;
-  const float *vz;
-  // the weights of cells z = 2n and 2n + 1
-  __device__ __forceinline__ float2 weights(int n) const {
-    const float2 pz = __ldg(reinterpret_cast<const float2 *>(vz) + n);
-    return make_float2(h.at(pz.x), h.at(pz.y));
-  }
-  __device__ __forceinline__ float2 load(const float2 *p, int n) const {
-    const float2 v = __ldcs(p), c = weights(n);
-    return make_float2(v.x * c.x, v.y * c.y);
-  }
+// The z pass. A CTA takes blocks of RP = 256 / T rows of one x-plane (T lanes transform a row, RowFft): the rows'
+// pairs come straight from HBM into registers (T consecutive pairs per load: 64 to 256 contiguous bytes), each
+// row is transformed within its warp, and the rows in shared memory are then split and stored transposed, RP * 8
+// contiguous bytes per kz. Rows kz > kzmax are beyond the top k-bin and are not written. L > 0: cells weighted
+// by h_Lm(r^); SP slots share their cells' weights (formed once per row and pair of slots).
+// What bounds it: HBM, at 0.88 of the copy rate. At 512^3 (four slots) it moves 4.3 GB in 0.72 ms, at 1024^3 34 GB
+// in 5.6 ms; the radix-8 stages in shared memory that it replaces took 0.93 and 9.3 ms (two more crossings of
+// shared memory, a block barrier per stage and twice the instructions). A weighted pass over two slots at 512^3:
+// 0.66 -> 0.38 ms, its rows above the top bin (a third of them for k < 0.62 of the Nyquist frequency) not written.
+template <int LOGM>
+struct ZfftShape {
+  typedef RowFft<LOGM> F;
+  static constexpr int M = F::N;
+  static constexpr int RP = ZR_THREADS / F::T;
+  static constexpr int PITCH = ((F::BUF > M ? F::BUF : M) + 1) | 1;  // odd: lanes across rows meet no bank conflict
+  static constexpr unsigned SMEM = 8u * (RP * PITCH + M + M / 2 + 1);
 };
 
-// The degree L is a compile-time constant, so the polynomial of each m is specialised.
-template <int L>
-struct ZrWeightLoad {
-  ZrWeight w;
-  __device__ __forceinline__ ZrWeightRow<L> row(int x, int y) const {
-    return ZrWeightRow<L>{HarmRow<L>(w.m, __ldg(w.vx + x), __ldg(w.vy + y)), w.vz};
-  }
-};
-
-// SP = 2 (an even number of slots): each block takes ZB / 2 rows of a pair of slots, whose cells share
-// their weights (the weights depend on the cell only).
-template <int ZB, int L, int SP>
-__global__ void __launch_bounds__(ZR_THREADS) k_zr2c_w(ZrGeo zg, BinTables t, const float *in, float2 *out,
-                                                       ZrWeightLoad<L> ld) {
+template <int LOGM, int L, int SP>
+__global__ void __launch_bounds__(ZR_THREADS, LOGM >= 9 ? 2 : (SP > 1 ? 3 : 4))
+    k_zfft(ZrGeo zg, BinTables t, const float *in, float2 *out, ZrWeight wt, int kzmax) {
+  typedef ZfftShape<LOGM> S;
+  typedef typename S::F F;
+  constexpr int M = S::M, T = F::T, R1 = F::R1, RP = S::RP;
   extern __shared__ __align__(16) unsigned char smz[];
-  constexpr int RS = ZB / SP;
-  const int M = 1 << zg.log2m;
-  float2 *sd = (float2 *)smz;  // [M][ZB + 1]
-  const ZrTables z = zr2c_load_tables(t, zg.log2m, smz + align16(8u * (unsigned)M * (ZB + 1)));
+  float2 *sd = (float2 *)smz;              // [RP][PITCH]
+  float2 *stw = sd + RP * S::PITCH;        // row twiddles
+  float2 *stp = stw + M;                   // exp(-2 pi i k / NZ), k <= M / 2
+  F::load_twiddles(stw, t.twz);
+  for (int k = threadIdx.x; k <= M / 2; k += ZR_THREADS) stp[k] = t.tpz[k];
+  const int tl = threadIdx.x % T, row = threadIdx.x / T;
+  float2 *srow = sd + row * S::PITCH;
+  const int orow = threadIdx.x % RP, ok = threadIdx.x / RP;  // output phase: row, first kz
   const int per_group = zg.nx * zg.nyb, nblk = per_group * (zg.ns / SP);
-  for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+  for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {  // (group of SP slots, x, block of RP rows)
     const int grp = blk / per_group, rem = blk - grp * per_group;
-    const int x = rem / zg.nyb, y0 = (rem - x * zg.nyb) * RS;
-    __syncthreads();
-    zr2c_block<ZB, ZrWeightLoad<L>, SP>(zg, z, in, out, sd, grp * SP, x, y0, ld);
+    const int x = rem / zg.nyb, y0 = (rem - x * zg.nyb) * RP, y = y0 + row, oy = y0 + orow;
+    float2 w[SP > 1 ? R1 : 1];
+    if constexpr (L > 0 && SP > 1) {
+      const HarmRow<L> h(wt.m, __ldg(wt.vx + x), __ldg(wt.vy + min(y, zg.ny - 1)));
+#pragma unroll
+      for (int q = 0; q < R1; q++) {
+        const float2 pz = __ldg(reinterpret_cast<const float2 *>(wt.vz) + tl + T * q);
+        w[q] = make_float2(h.at(pz.x), h.at(pz.y));
+      }
+    }
+#pragma unroll 1
+    for (int s = 0; s < SP; s++) {
+      const int sl = grp * SP + s;
+      float2 v[R1];
+      const float2 *rp = reinterpret_cast<const float2 *>(in + sl * zg.in_slot + (long long)x * zg.slice +
+                                                          (long long)min(y, zg.ny - 1) * zg.row) + tl;
+#pragma unroll
+      for (int q = 0; q < R1; q++) v[q] = __ldcs(rp + T * q);
+      if (SP == 1 && L == 0) {
+        // the CTA's next block is RP contiguous padded rows: one bulk prefetch into L2 while this one runs
+        const int nb = blk + (int)gridDim.x;
+        if (threadIdx.x == 0 && nb < nblk) {
+          const int sl2 = nb / per_group, rem2 = nb - sl2 * per_group;
+          const int x2 = rem2 / zg.nyb, y2 = (rem2 - x2 * zg.nyb) * RP;
+          const float *nxt = in + sl2 * zg.in_slot + (long long)x2 * zg.slice + (long long)y2 * zg.row;
+          const unsigned bytes = ((unsigned)(min(RP, zg.ny - y2) * zg.row) * 4u) & ~15u;
+          if (bytes && (((unsigned long long)nxt & 15ull) == 0))
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(nxt), "r"(bytes) : "memory");
+        }
+      }
+      if constexpr (L > 0) {
+        if constexpr (SP > 1) {
+#pragma unroll
+          for (int q = 0; q < R1; q++) v[q] = make_float2(v[q].x * w[q].x, v[q].y * w[q].y);
+        } else {
+          const HarmRow<L> h(wt.m, __ldg(wt.vx + x), __ldg(wt.vy + min(y, zg.ny - 1)));
+#pragma unroll
+          for (int q = 0; q < R1; q++) {
+            const float2 pz = __ldg(reinterpret_cast<const float2 *>(wt.vz) + tl + T * q);
+            v[q] = make_float2(v[q].x * h.at(pz.x), v[q].y * h.at(pz.y));
+          }
+        }
+      }
+      __syncthreads();  // tables written; the previous rows' output has read sd
+      F::run(v, srow, stw, tl);
+#pragma unroll
+      for (int u = 0; u < F::G; u++)
+#pragma unroll
+        for (int r = 0; r < T; r++) srow[tl + T * u + R1 * r] = v[u * T + r];
+      __syncthreads();
+      // real-input split and transposed store, X[k] and X[M-k] from the same pair: with
+      // A = Z[k] + conj Z[M-k], B = Z[k] - conj Z[M-k] and w^M = -1, X[k] = (A + (-i) w^k B) / 2 and
+      // X[M-k] = (conj A + (-i) conj(w^k B)) / 2.
+      if (oy < zg.ny) {
+        const float2 *zr = sd + orow * S::PITCH;
+        float2 *dst = out + sl * zg.out_slot + (long long)x * zg.nzc * zg.ny + oy;
+        for (int k = ok; k <= M / 2; k += T) {
+          const float2 zk = zr[k], zm = zr[(M - k) & (M - 1)];
+          const float2 A = make_float2(zk.x + zm.x, zk.y - zm.y);
+          const float2 B = make_float2(zk.x - zm.x, zk.y + zm.y);
+          const float2 wB = cmulf(stp[k], B);
+          if (k <= kzmax) dst[(long long)k * zg.ny] = make_float2(0.5f * (A.x + wB.y), 0.5f * (A.y - wB.x));
+          if (2 * k != M && M - k <= kzmax)
+            dst[(long long)(M - k) * zg.ny] = make_float2(0.5f * (A.x - wB.y), -0.5f * (A.y + wB.x));
+        }
+      }
+    }
   }
 }
 
-template <int ZB, int L, int SP>
-static void launch_zr2c_w_sp(cudaStream_t s, ZrGeo zg, const BinTables &t, int nslot, const float *in,
-                             float2 *out, const ZrWeight &w) {
-  const int M = 1 << zg.log2m;
-  zg.nyb = (zg.ny + ZB / SP - 1) / (ZB / SP);
-  const size_t smem = align16(8u * (unsigned)M * (ZB + 1)) + zr2c_tables_bytes(zg.log2m);
-  cudaFuncSetAttribute(k_zr2c_w<ZB, L, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int LOGM, int L, int SP>
+static void launch_zfft_t(cudaStream_t s, ZrGeo zg, const BinTables &t, int nslot, const float *in, float2 *out,
+                          const ZrWeight &w, int kzmax) {
+  typedef ZfftShape<LOGM> S;
+  zg.nyb = (zg.ny + S::RP - 1) / S::RP;
+  const size_t smem = S::SMEM;
+  cudaFuncSetAttribute(k_zfft<LOGM, L, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 1, dev = 0, nsm = 152;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zr2c_w<ZB, L, SP>, ZR_THREADS, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zfft<LOGM, L, SP>, ZR_THREADS, smem);
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const long long nblk = (long long)zg.nx * zg.nyb * (nslot / SP);
   long long grid = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
   if (grid > nblk) grid = nblk;
-  k_zr2c_w<ZB, L, SP><<<(unsigned)grid, ZR_THREADS, smem, s>>>(zg, t, in, out, ZrWeightLoad<L>{w});
+  k_zfft<LOGM, L, SP><<<(unsigned)grid, ZR_THREADS, smem, s>>>(zg, t, in, out, w, kzmax);
 }
 
-template <int ZB, int L>
-static void launch_zr2c_w_l(cudaStream_t s, const ZrGeo &zg, const BinTables &t, int nslot, const float *in,
-                            float2 *out, const ZrWeight &w) {
-  if (nslot % 2 == 0 && (zg.in_slot % 2) == 0) launch_zr2c_w_sp<ZB, L, 2>(s, zg, t, nslot, in, out, w);
-  else launch_zr2c_w_sp<ZB, L, 1>(s, zg, t, nslot, in, out, w);
-}
-
-template <int ZB>
-static void launch_zr2c_w_t(cudaStream_t s, const ZrGeo &zg, const BinTables &t, int nslot, const float *in,
-                            float2 *out, const ZrWeight &w) {
+// Two slots a thread share the weights they read their cells with while a row's values and its weights fit the
+// registers (M <= 256).
+template <int LOGM>
+static void launch_zfft_m(cudaStream_t s, const ZrGeo &zg, const BinTables &t, int nslot, const float *in, float2 *out,
+                          const ZrWeight &w, int kzmax) {
+  constexpr int SP = LOGM <= 8 ? 2 : 1;
+  const bool two = SP == 2 && nslot % 2 == 0;
   switch (w.l) {
-    case 1: launch_zr2c_w_l<ZB, 1>(s, zg, t, nslot, in, out, w); break;
-    case 2: launch_zr2c_w_l<ZB, 2>(s, zg, t, nslot, in, out, w); break;
-    case 3: launch_zr2c_w_l<ZB, 3>(s, zg, t, nslot, in, out, w); break;
-    default: launch_zr2c_w_l<ZB, 4>(s, zg, t, nslot, in, out, w); break;
+    case 0: launch_zfft_t<LOGM, 0, 1>(s, zg, t, nslot, in, out, w, kzmax); break;
+    case 1: two ? launch_zfft_t<LOGM, 1, SP>(s, zg, t, nslot, in, out, w, kzmax)
+                : launch_zfft_t<LOGM, 1, 1>(s, zg, t, nslot, in, out, w, kzmax); break;
+    case 2: two ? launch_zfft_t<LOGM, 2, SP>(s, zg, t, nslot, in, out, w, kzmax)
+                : launch_zfft_t<LOGM, 2, 1>(s, zg, t, nslot, in, out, w, kzmax); break;
+    case 3: two ? launch_zfft_t<LOGM, 3, SP>(s, zg, t, nslot, in, out, w, kzmax)
+                : launch_zfft_t<LOGM, 3, 1>(s, zg, t, nslot, in, out, w, kzmax); break;
+    default: two ? launch_zfft_t<LOGM, 4, SP>(s, zg, t, nslot, in, out, w, kzmax)
+                 : launch_zfft_t<LOGM, 4, 1>(s, zg, t, nslot, in, out, w, kzmax); break;
   }
+}
+
+static void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+                        long long in_slot, int row, float2 *out, long long out_slot, const ZrWeight &w,
+                        long long *launches) {
+  const ZrGeo zg = zr2c_geo(bp, nslot, in_slot, row, out_slot);
+  switch (zg.log2m) {
+    case 4: launch_zfft_m<4>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+    case 5: launch_zfft_m<5>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+    case 6: launch_zfft_m<6>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+    case 7: launch_zfft_m<7>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+    case 8: launch_zfft_m<8>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+    case 9: launch_zfft_m<9>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+    default: launch_zfft_m<10>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
+  }
+  (*launches)++;
+}
+
+void launch_zr2c(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+                 long long in_slot, int row, float2 *out, long long out_slot, long long *launches) {
+  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{nullptr, nullptr, nullptr, 0, 0}, launches);
 }
 
 void launch_zr2c_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                           long long in_slot, int row, float2 *out, long long out_slot, const float *vx,
                           const float *vy, const float *vz, int l, int m, long long *launches) {
-  ZrGeo zg = zr2c_geo(bp, nslot, in_slot, row, out_slot);
-  const ZrWeight ld{vx, vy, vz, l, m};
-  if (bp.nz <= 512) {
-    zg.nyb = (bp.ny + 15) / 16;
-    launch_zr2c_w_t<16>(s, zg, t, nslot, in, out, ld);
-  } else {
-    zg.nyb = (bp.ny + 7) / 8;
-    launch_zr2c_w_t<8>(s, zg, t, nslot, in, out, ld);
-  }
-  (*launches)++;
+  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{vx, vy, vz, l, m}, launches);
 }
 
 // ------------------------------------------------------------ z and y axes in one launch (FP32)
@@ -1650,35 +1634,6 @@ bool zr2c_supported(const BinParams &bp) {
   return bp.nz >= 32 && bp.nz <= 2048 && (bp.nz & (bp.nz - 1)) == 0;
 }
 
-template <int ZB>
-static void launch_zr2c_t(cudaStream_t s, const ZrGeo &zg, const BinTables &t, int nslot, const float *in,
-                          float2 *out) {
-  const int M = 1 << zg.log2m;
-  const size_t smem = align16(8u * (unsigned)M * (ZB + 1)) + zr2c_tables_bytes(zg.log2m);
-  cudaFuncSetAttribute(k_zr2c<ZB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 1, dev = 0, nsm = 152;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zr2c<ZB>, ZR_THREADS, smem);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long nblk = (long long)zg.nx * zg.nyb * nslot;
-  long long grid = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
-  if (grid > nblk) grid = nblk;
-  k_zr2c<ZB><<<(unsigned)grid, ZR_THREADS, smem, s>>>(zg, t, in, out);
-}
-
-void launch_zr2c(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
-                 long long in_slot, int row, float2 *out, long long out_slot, long long *launches) {
-  ZrGeo zg = zr2c_geo(bp, nslot, in_slot, row, out_slot);
-  if (bp.nz <= 512) {  // 16 rows per CTA: 128-byte segments per kz
-    zg.nyb = (bp.ny + 15) / 16;
-    launch_zr2c_t<16>(s, zg, t, nslot, in, out);
-  } else {  // 8 rows per CTA keeps the shared rows within 80 KB
-    zg.nyb = (bp.ny + 7) / 8;
-    launch_zr2c_t<8>(s, zg, t, nslot, in, out);
-  }
-  (*launches)++;
-}
-
 bool zy_supported(const BinParams &bp, const BinTables &t) {
   return zr2c_supported(bp) && t.twy && bp.ny >= 16 && bp.ny <= 2048 && (bp.ny & (bp.ny - 1)) == 0;
 }
@@ -1809,6 +1764,14 @@ void bin_params_kguess(BinParams &bp, const capow_params &p) {
   bp.lg = p.OutputLog ? 1 : 0;
   bp.kscale = (float)(2.0 * M_PI / bw);
   bp.koff = (float)(-p.Mink / bw);
+  // the top edge in k: Maxk (10^Maxk for log bins) or the smallest Nyquist frequency (src/main.c:320-325, 369-375)
+  double top = p.OutputLog ? pow(10.0, p.Maxk) : p.Maxk;
+  const double n[3] = {(double)p.NX, (double)p.NY, (double)p.NZ};
+  const double l[3] = {p.XMAX - p.XMIN, p.YMAX - p.YMIN, p.ZMAX - p.ZMIN};
+  for (int a = 0; a < 3; a++) top = fmin(top, M_PI * n[a] / l[a]);
+  // rows beyond it (with a whole row to spare) have no mode in any bin
+  const double kz = top * l[2] / (2.0 * M_PI) + 2.0;
+  bp.kzmax = kz < 0.0 ? 0 : (kz < (double)(p.NZ / 2) ? (int)kz : p.NZ / 2);
 }
 
 void launch_mode_counts(cudaStream_t s, const BinParams &bp, const BinTables &t, unsigned long long *nmodes,

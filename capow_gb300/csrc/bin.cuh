@@ -59,6 +59,7 @@ struct BinParams {
   // starts the walk over the safe FP32 edges, so its rounding does not matter.
   float kscale, koff;
   int lg;
+  int kzmax;  // kz rows beyond this one lie above the top bin edge: no stage needs them
 };
 
 // bin in [-1, NK] of an exact s: E[b+1] <= s < E[b+2]
@@ -80,7 +81,7 @@ __device__ __forceinline__ int herm_nm(int i, int j, int k, int xhalf) {
   return (i != xhalf) ? 1 : 2;
 }
 
-// Fill kscale, koff and lg of bp for a run's k binning.
+// Fill kscale, koff, lg and kzmax of bp for a run's k binning.
 void bin_params_kguess(BinParams &bp, const capow_params &p);
 
 // Host: exact k-bin of one |k|^2 value s, following src/main.c:355, 369-375.

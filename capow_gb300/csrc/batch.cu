@@ -282,7 +282,7 @@ int setup_batch(BatchState *b, const capow_mock *mocks, int nmocks, const capow_
     m.bp.out2d = p.Output2D;
     m.bp.fx_step = (float)(1.0 / ((float)p.NX * m.g.dx));
     bin_params_kguess(m.bp, p);
-    if (c->fused && !xbin_plan(m.bp, c->nslot, m.xg, c->xtr)) {  // this mock's bins do not fit the pass
+    if (c->fused && !(c->blk ? xrow_plan(m.bp, c->bt, c->nslot, m.xg) : xbin_plan(m.bp, c->nslot, m.xg, c->xtr))) {  // this mock's bins do not fit the pass
       b->status0[i] = CAPOW_ENOTSUP;
       b->ctx_of[i] = nullptr;
       continue;

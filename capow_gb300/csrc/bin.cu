@@ -21,6 +21,7 @@
 #include "bin.cuh"
 #include "fft_dev.cuh"
 #include "harm.cuh"
+#include "launch.cuh"
 #include "paint.cuh"
 
 // ------------------------------------------------------------------------------------ host side
@@ -1133,13 +1134,14 @@ template <int LOGM>
 struct ZfftShape {
   typedef RowFft<LOGM> F;
   static constexpr int M = F::N;
-  static constexpr int RP = ZR_THREADS / F::T;
+  static constexpr int THREADS = LOGM == 9 ? 512 : ZR_THREADS;  // 16 rows of 512
+  static constexpr int RP = THREADS / F::T;
   static constexpr int PITCH = ((F::BUF > M ? F::BUF : M) + 1) | 1;  // odd: lanes across rows meet no bank conflict
   static constexpr unsigned SMEM = 8u * (RP * PITCH + M + M / 2 + 1);
 };
 
 template <int LOGM, int L, int SP>
-__global__ void __launch_bounds__(ZR_THREADS, LOGM >= 9 ? 2 : (SP > 1 ? 3 : 4))
+__global__ void __launch_bounds__(ZfftShape<LOGM>::THREADS, LOGM >= 9 ? 2 : (SP > 1 ? 3 : 4))
     k_zfft(ZrGeo zg, BinTables t, const float *in, float2 *out, ZrWeight wt, int kzmax) {
   typedef ZfftShape<LOGM> S;
   typedef typename S::F F;
@@ -1149,7 +1151,7 @@ __global__ void __launch_bounds__(ZR_THREADS, LOGM >= 9 ? 2 : (SP > 1 ? 3 : 4))
   float2 *stw = sd + RP * S::PITCH;        // row twiddles
   float2 *stp = stw + M;                   // exp(-2 pi i k / NZ), k <= M / 2
   F::load_twiddles(stw, t.twz);
-  for (int k = threadIdx.x; k <= M / 2; k += ZR_THREADS) stp[k] = t.tpz[k];
+  for (int k = threadIdx.x; k <= M / 2; k += S::THREADS) stp[k] = t.tpz[k];
   const int tl = threadIdx.x % T, row = threadIdx.x / T;
   float2 *srow = sd + row * S::PITCH;
   const int orow = threadIdx.x % RP, ok = threadIdx.x / RP;  // output phase: row, first kz
@@ -1202,9 +1204,7 @@ __global__ void __launch_bounds__(ZR_THREADS, LOGM >= 9 ? 2 : (SP > 1 ? 3 : 4))
       __syncthreads();  // tables written; the previous rows' output has read sd
       F::run(v, srow, stw, tl);
 #pragma unroll
-      for (int u = 0; u < F::G; u++)
-#pragma unroll
-        for (int r = 0; r < T; r++) srow[tl + T * u + R1 * r] = v[u * T + r];
+      for (int j = 0; j < R1; j++) srow[F::freq(tl, j)] = v[j];
       __syncthreads();
       // real-input split and transposed store, X[k] and X[M-k] from the same pair: with
       // A = Z[k] + conj Z[M-k], B = Z[k] - conj Z[M-k] and w^M = -1, X[k] = (A + (-i) w^k B) / 2 and
@@ -1232,15 +1232,11 @@ static void launch_zfft_t(cudaStream_t s, ZrGeo zg, const BinTables &t, int nslo
   typedef ZfftShape<LOGM> S;
   zg.nyb = (zg.ny + S::RP - 1) / S::RP;
   const size_t smem = S::SMEM;
-  cudaFuncSetAttribute(k_zfft<LOGM, L, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 1, dev = 0, nsm = 152;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zfft<LOGM, L, SP>, ZR_THREADS, smem);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int resident = resident_ctas((const void *)k_zfft<LOGM, L, SP>, S::THREADS, smem);
   const long long nblk = (long long)zg.nx * zg.nyb * (nslot / SP);
-  long long grid = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
+  long long grid = resident;
   if (grid > nblk) grid = nblk;
-  k_zfft<LOGM, L, SP><<<(unsigned)grid, ZR_THREADS, smem, s>>>(zg, t, in, out, w, kzmax);
+  k_zfft<LOGM, L, SP><<<(unsigned)grid, S::THREADS, smem, s>>>(zg, t, in, out, w, kzmax);
 }
 
 // Two slots a thread share the weights they read their cells with while a row's values and its weights fit the
@@ -1265,8 +1261,12 @@ static void launch_zfft_m(cudaStream_t s, const ZrGeo &zg, const BinTables &t, i
 
 static void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                         long long in_slot, int row, float2 *out, long long out_slot, const ZrWeight &w,
-                        long long *launches) {
-  const ZrGeo zg = zr2c_geo(bp, nslot, in_slot, row, out_slot);
+                        long long *launches, int x0, int nx) {
+  ZrGeo zg = zr2c_geo(bp, nslot, in_slot, row, out_slot);
+  if (nx >= 0) {
+    zg.nx = nx;
+    in += (long long)x0 * zg.slice;
+  }
   switch (zg.log2m) {
     case 4: launch_zfft_m<4>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
     case 5: launch_zfft_m<5>(s, zg, t, nslot, in, out, w, bp.kzmax); break;
@@ -1280,14 +1280,15 @@ static void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t,
 }
 
 void launch_zr2c(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
-                 long long in_slot, int row, float2 *out, long long out_slot, long long *launches) {
-  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{nullptr, nullptr, nullptr, 0, 0}, launches);
+                 long long in_slot, int row, float2 *out, long long out_slot, long long *launches, int x0, int nx) {
+  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{nullptr, nullptr, nullptr, 0, 0}, launches, x0,
+              nx);
 }
 
 void launch_zr2c_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                           long long in_slot, int row, float2 *out, long long out_slot, const float *vx,
                           const float *vy, const float *vz, int l, int m, long long *launches) {
-  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{vx, vy, vz, l, m}, launches);
+  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{vx, vy, vz, l, m}, launches, 0, -1);
 }
 
 // ------------------------------------------------------------ z and y axes in one launch (FP32)
@@ -1646,12 +1647,8 @@ static void launch_zy_t(cudaStream_t s, const ZyGeo &yg, const BinTables &t, con
   const unsigned M = 1u << yg.zg.log2m, ny = 1u << yg.log2ny;
   const unsigned zdata = zy_zdata_bytes(yg.zg.log2m, ZB), ydata = align16(8u * ZY_KB * (ny + ny / 8));
   const size_t smem = (zdata > ydata ? zdata : ydata) + zr2c_tables_bytes(yg.zg.log2m) + zy_ytables_bytes(yg.log2ny);
-  cudaFuncSetAttribute(k_zy<ZB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 1, dev = 0, nsm = 152;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zy<ZB>, ZR_THREADS, smem);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  long long grid = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
+  const int resident = resident_ctas((const void *)k_zy<ZB>, ZR_THREADS, smem);
+  long long grid = resident;
   if (grid > yg.nitems) grid = yg.nitems;
   k_zy<ZB><<<(unsigned)grid, ZR_THREADS, smem, s>>>(yg, t, in, out, ctr, st);
 }
@@ -1721,13 +1718,8 @@ static void launch_xbin_t(cudaStream_t s, const BinParams &bp, const BinTables &
                           void *const slots[4], const double *dcv, double *bins) {
   constexpr int NP = NF == 1 ? 1 : 4, NL = ODD ? 5 : 3;
   const size_t smem = xbin_smem_layout(xg.log2n, xg.ncol, NP, NL, bp.nk, xg.nbc).total;
-  cudaFuncSetAttribute(k_xfft_bin<NF, IL, ODD, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_xfft_bin<NF, IL, ODD, PM>, XBIN_THREADS, smem);
-  int dev = 0, nsm = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  int grid = (per_sm > 0 ? per_sm : 1) * nsm;
+  const int resident = resident_ctas((const void *)k_xfft_bin<NF, IL, ODD, PM>, XBIN_THREADS, smem);
+  int grid = resident;
   if (grid > xg.nblocks) grid = xg.nblocks;
   k_xfft_bin<NF, IL, ODD, PM><<<grid, XBIN_THREADS, smem, s>>>(bp, t, xg, (const float2 *)slots[0],
                                                                 (const float2 *)slots[1], (const float2 *)slots[2],
@@ -1771,6 +1763,9 @@ void bin_params_kguess(BinParams &bp, const capow_params &p) {
   for (int a = 0; a < 3; a++) top = fmin(top, M_PI * n[a] / l[a]);
   // rows beyond it (with a whole row to spare) have no mode in any bin
   const double kz = top * l[2] / (2.0 * M_PI) + 2.0;
+  bp.fy_step = (float)(1.0 / l[1]);
+  bp.fz_step = (float)(1.0 / l[2]);
+  bp.ftop2 = top > 0.0 ? (float)(top / (2.0 * M_PI) * (top / (2.0 * M_PI))) : 0.0f;
   bp.kzmax = kz < 0.0 ? 0 : (kz < (double)(p.NZ / 2) ? (int)kz : p.NZ / 2);
 }
 

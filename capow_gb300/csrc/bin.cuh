@@ -38,7 +38,8 @@ struct BinTables {
 // Geometry of the fused x-axis FFT + binning pass (k_xfft_bin): blocks of `ncol` columns of the
 // (y, z)-transformed grids, `kc` consecutive "inner" indices of one "outer" index in each of the
 // nslot grids. Layout [NX][outer][inner]: tr = 0, [NX][NY][NZ/2+1] (outer ky, inner kz, after the
-// cuFFT 2-D transform); tr = 1, [NX][NZ/2+1][NY] (outer kz, inner ky, after k_zr2c and the y pass).
+// cuFFT 2-D transform); tr = 1, [NX][NZ/2+1][NY] (outer kz, inner ky, after k_zr2c and the y pass); tr = 2,
+// [NZ/2+1][NY][NX] (k_yfft and k_xrow_bin, xbin.cu).
 struct XbinGeo {
   int log2n, ncol, log2ncol, kc, log2kc, nkb, nblocks;
   int tr, n_outer, n_inner;
@@ -60,6 +61,8 @@ struct BinParams {
   float kscale, koff;
   int lg;
   int kzmax;  // kz rows beyond this one lie above the top bin edge: no stage needs them
+  float fy_step, fz_step;  // y and z frequency spacings
+  float ftop2;             // |f|^2 of the top bin edge (to FP32)
 };
 
 // bin in [-1, NK] of an exact s: E[b+1] <= s < E[b+2]
@@ -81,7 +84,7 @@ __device__ __forceinline__ int herm_nm(int i, int j, int k, int xhalf) {
   return (i != xhalf) ? 1 : 2;
 }
 
-// Fill kscale, koff, lg and kzmax of bp for a run's k binning.
+// Fill kscale, koff, lg, kzmax, the y and z spacings and ftop2 of bp for a run's k binning.
 void bin_params_kguess(BinParams &bp, const capow_params &p);
 
 // Host: exact k-bin of one |k|^2 value s, following src/main.c:355, 369-375.
@@ -128,9 +131,20 @@ void launch_zy(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslo
 void launch_zr2c_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                           long long in_slot, int row, float2 *out, long long out_slot, const float *vx,
                           const float *vy, const float *vz, int l, int m, long long *launches);
+// (x0, nx: only those planes, out then starting at plane x0)
 void launch_zr2c(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
-                 long long in_slot, int row, float2 *out, long long out_slot, long long *launches);
+                 long long in_slot, int row, float2 *out, long long out_slot, long long *launches, int x0 = 0,
+                 int nx = -1);
 void launch_xbin(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg, void *const slots[4],
+                 const double *dcv, double *bins, long long *launches);
+// The blocked path (xbin.cu; power-of-two NX, NY, NZ): its plan (false where k_xbin's layouts are used), the y axis
+// of planes x0 .. x0 + nx - 1 from the z pass's layout into the blocked one (not in the launch count: it stands where
+// the other layouts have a library transform), and the fused x axis + binning.
+bool yfft_supported(const BinParams &bp, const BinTables &t);
+bool xrow_plan(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg);
+void launch_yfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, int x0, int nx,
+                 const float2 *in, long long in_slot, float2 *out, long long out_slot);
+void launch_xrow(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg, void *const slots[4],
                  const double *dcv, double *bins, long long *launches);
 // DC corrections: dcv[slot] = painted sum (minus NGRID for mean-subtracted field A slots)
 void launch_dc_prepare(cudaStream_t s, const void *st, int deterministic, int nslot, int nfields, int mean_sub_a,

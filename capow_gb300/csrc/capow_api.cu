@@ -8,6 +8,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "ctx.cuh"
@@ -247,6 +248,30 @@ extern "C" int capow_create(const capow_params *p, const capow_options *opt, cap
   const bool want_fused = !f64 && o.fft_path != CAPOW_FFT_3D && c->bt.twx;
   const long long yrows = (long long)c->nslot * p->NX * bp.nzc;
   const bool tr = want_fused && c->bt.twz && zr2c_supported(bp) && yrows <= 0x7fffffffLL;
+  if (tr && o.fft_path == CAPOW_FFT_AUTO && xrow_plan(bp, c->bt, c->nslot, c->xg)) {
+    // power-of-two NY too: the blocked path. Its z and y passes run on up to 4 GB of planes at a time, so that a
+    // large grid needs no third grid-sized buffer. (Each pair of launches costs about 20 us of ramps: at 512^3, runs
+    // of planes that would stay in L2 between the passes took 1.76 ms at 64 MB and 2.7 ms at 32 MB, against 1.43 ms
+    // for one of each.)
+    const long long plane = (long long)bp.nzc * p->NY;
+    // (a multiple of 64: the y pass writes runs of 16 planes)
+    c->planes = (int)std::min<long long>(p->NX, std::max<long long>(1, (4LL << 30) / (8 * plane * c->nslot) / 64) * 64);
+    c->tslot = plane * c->planes;
+    c->uslot = plane * p->NX;
+    void *tb = nullptr, *ub = nullptr;
+    if (cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess &&
+        cudaMalloc(&ub, sizeof(float2) * (size_t)c->uslot * c->nslot) == cudaSuccess) {
+      c->allocs.push_back(tb);
+      c->allocs.push_back(ub);
+      c->tbuf = (float2 *)tb;
+      c->ubuf = (float2 *)ub;
+      c->fused = c->xtr = c->blk = true;
+      c->plan_ok = true;  // the context is complete (no cuFFT plan on this path)
+      return CAPOW_OK;
+    }
+    if (tb) cudaFree(tb);
+    (void)cudaGetLastError();  // no room: the layouts below
+  }
   c->fused = want_fused && xbin_plan(bp, c->nslot, c->xg, tr);
   if (c->fused && tr) {
     // the transposed layout needs a second grid-sized buffer and a cuFFT workspace; when the device
@@ -675,7 +700,15 @@ int enqueue_power_kernels(capow_ctx *c) {
                     c->bp.mean_sub_a, c->fixed_scale, c->dcv, &c->launches);
   if (c->fused) {
     void *slots[4];
-    if (c->xtr && c->zy) {
+    if (c->blk) {
+      for (int x0 = 0; x0 < c->p.NX; x0 += c->planes) {
+        const int nx = std::min(c->planes, c->p.NX - x0);
+        launch_zr2c(c->stream, c->bp, c->bt, c->nslot, (const float *)c->grid_base, (long long)c->grid_elems, c->g.row,
+                    c->tbuf, c->tslot, &c->launches, x0, nx);
+        launch_yfft(c->stream, c->bp, c->bt, c->nslot, x0, nx, c->tbuf, c->tslot, c->ubuf, c->uslot);
+      }
+      for (int k = 0; k < 4; k++) slots[k] = k < c->nslot ? (void *)(c->ubuf + c->uslot * k) : nullptr;
+    } else if (c->xtr && c->zy) {
       launch_zy(c->stream, c->bp, c->bt, c->nslot, (const float *)c->grid_base, (long long)c->grid_elems, c->g.row,
                 c->tbuf, c->tslot, c->zy_ctr, c->st, c->zy_stall, &c->launches);
       CK(c, cudaGetLastError());
@@ -694,7 +727,8 @@ int enqueue_power_kernels(capow_ctx *c) {
     if (!c->quiet) CK(c, cudaEventRecord(c->ev[2], c->stream));
     const int nk = c->p.NK;
     CK(c, cudaMemsetAsync(c->bins, 0, sizeof(double) * NPROD * 5 * nk, c->stream));
-    launch_xbin(c->stream, c->bp, c->bt, c->xg, slots, c->dcv, c->bins, &c->launches);
+    if (c->blk) launch_xrow(c->stream, c->bp, c->bt, c->xg, slots, c->dcv, c->bins, &c->launches);
+    else launch_xbin(c->stream, c->bp, c->bt, c->xg, slots, c->dcv, c->bins, &c->launches);
     CK(c, cudaGetLastError());
     if (!c->quiet) CK(c, cudaEventRecord(c->ev[3], c->stream));
     return CAPOW_OK;

@@ -46,7 +46,13 @@ struct capow_ctx {
   long long tslot;  // complex values per slot of tbuf
   cufftHandle yplan;
   bool yplan_ok;
-  // power-of-two NY as well: the z pass and the y axis in one launch (k_zy) instead of k_zr2c + yplan;
+  // blocked fused path (power-of-two NX, NY and NZ): the z pass of `planes` x-planes at a time into tbuf, the y axis
+  // from there into ubuf, [NZ/2+1][NY][NX] per slot, and k_xrow_bin on ubuf
+  bool blk;
+  int planes;
+  float2 *ubuf;
+  long long uslot;
+  // opt-in (CAPOW_FFT_ONE_LAUNCH): power-of-two NY as well: the z pass and the y axis in one launch (k_zy) instead of k_zr2c + yplan;
   // zy_ctr holds its work-queue and per-plane counters
   bool zy;
   unsigned *zy_ctr;

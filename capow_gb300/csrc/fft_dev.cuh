@@ -3,8 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Packed FP32 additions: one instruction per complex sum, rounded as the scalar ones are.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -56,7 +57,9 @@ __device__ __forceinline__ float2 mul_w32(float2 v, int k) {
     case 8: return cmul_mi(v);
     case 9: return cmulf(v, make_float2(-s1, -c1));
     case 10: return cmulf(v, make_float2(-s2, -c2));
+    case 11: return cmulf(v, make_float2(-s3, -c3));
     case 12: return make_float2((v.y - v.x) * h, -(v.x + v.y) * h);
+    case 13: return cmulf(v, make_float2(-c3, -s3));
     case 14: return cmulf(v, make_float2(-c2, -s2));
     case 15: return cmulf(v, make_float2(-c1, -s1));
     case 18: return cmulf(v, make_float2(-c2, s2));
@@ -96,18 +99,24 @@ __device__ __forceinline__ void dft(float2 *a) {
   }
 }
 
-// A row of N = 2^LOGN complex values by T = N / R1 lanes of one warp: lane t holds x[t + T q], q < R1. An R1-point
-// DFT per lane, twiddles, one exchange through the row's shared buffer, then R1 / T DFTs of T points per lane:
-// G groups u of output frequencies p + R1 r, p = t + T u, r < T, in v[u * T + r]. Against three radix-8 stages a
-// row crosses shared memory once instead of twice, and lanes of one warp exchange without a block barrier.
+// A row of N = 2^LOGN complex values by T lanes of one warp: lane t holds x[t + T q], q < R1, R1 = N / T. An R1-point
+// DFT per lane, twiddles, one exchange through the row's shared buffer, then R1 DFTs of T points, R1 / T per lane
+// (for N = 512, where 16 values a lane leave T = 32 > R1, half of one: two lanes take the even and the odd outputs
+// of one, 16 points each after a first radix-2 step). Output j of lane t is frequency freq(t, j). Against three radix-8 stages a row crosses
+// shared memory once instead of twice, and the lanes of one warp exchange without a block barrier. 16 values a lane
+// fit 64 registers, 32 (N = 1024) 128.
 template <int LOGN>
 struct RowFft {
   static constexpr int N = 1 << LOGN;
-  static constexpr int R1 = LOGN >= 9 ? 32 : (LOGN >= 7 ? 16 : (LOGN >= 5 ? 8 : 4));
+  static constexpr int R1 = LOGN == 10 ? 32 : (LOGN >= 7 ? 16 : (LOGN >= 5 ? 8 : 4));
   static constexpr int T = N / R1;
-  static constexpr int G = R1 / T;
   static constexpr int BUF = R1 * (T + 1);  // values of the exchange buffer
-  static_assert(LOGN >= 4 && LOGN <= 10 && G >= 1 && T * G == R1, "row length");
+  static_assert(LOGN >= 4 && LOGN <= 10 && T <= 32, "row length");
+
+  __device__ static __forceinline__ int freq(int t, int j) {
+    if constexpr (T > R1) return (t & (R1 - 1)) + R1 * (2 * j + t / R1);
+    else return t + T * (j / T) + R1 * (j % T);
+  }
 
   // tw[p * T + t] = exp(-2 pi i t p / N) (shared memory); buf: the row's BUF values, free on entry and exit
   __device__ static __forceinline__ void run(float2 *v, float2 *buf, const float2 *tw, int t) {
@@ -117,13 +126,28 @@ struct RowFft {
 #pragma unroll
     for (int p = 0; p < R1; p++) buf[p * (T + 1) + t] = v[p];
     __syncwarp();
+    if constexpr (T > R1) {  // N = 512: DFT p by lanes p and p + 16: outputs 2 r + h, h = 0 or 1
+      static_assert(T == 32 && R1 == 16, "split second stage");
+      const int p = t & 15, h = t >> 4;
+      const float sg = h ? -1.0f : 1.0f;
 #pragma unroll
-    for (int u = 0; u < G; u++)
+      for (int r = 0; r < 16; r++) {
+        const float2 lo = buf[p * 33 + r], hi = buf[p * 33 + r + 16];
+        const float2 d = __ffma2_rn(hi, make_float2(sg, sg), lo);
+        v[r] = r == 0 ? d : (h ? mul_w32(d, r) : d);
+      }
+      __syncwarp();
+      dft<16>(v);
+    } else {
+      constexpr int G = R1 / T;
 #pragma unroll
-      for (int r = 0; r < T; r++) v[u * T + r] = buf[(t + T * u) * (T + 1) + r];
-    __syncwarp();
+      for (int u = 0; u < G; u++)
 #pragma unroll
-    for (int u = 0; u < G; u++) dft<T>(v + u * T);
+        for (int r = 0; r < T; r++) v[u * T + r] = buf[(t + T * u) * (T + 1) + r];
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < G; u++) dft<T>(v + u * T);
+    }
   }
 
   // the twiddle table from a table of exp(-2 pi i q / N), q < N

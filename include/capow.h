@@ -274,7 +274,8 @@ int capow_stage_ms(capow_ctx *ctx, float *paint_ms, float *fft_ms, float *bin_ms
  * CAPOW_ESTATE on FP64 contexts or before an FP32 paint. */
 int capow_tile_kernel_ms(capow_ctx *ctx, float *ms, int64_t *records);
 
-/* total number of kernels this library launched on the context since creation */
+/* total number of kernels this library launched on the context since creation (the axis transforms by
+ * cuFFT, and the y-axis pass that stands in their place on the blocked layout, are not counted) */
 int64_t capow_kernel_launches(const capow_ctx *ctx);
 
 void capow_destroy(capow_ctx *ctx);

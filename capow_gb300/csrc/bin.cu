@@ -16,6 +16,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "bin.cuh"
@@ -236,9 +237,10 @@ __device__ __forceinline__ int exact_mubin(const BinParams &bp, const BinTables 
   return mb;
 }
 
-// One-time mode counts (Nmodes, Nmodes_2D): exact for every mode.
-__global__ void __launch_bounds__(256) k_mode_counts(BinParams bp, BinTables t, unsigned long long *nm,
-                                                     unsigned long long *nm2d) {
+// Mode counts with 2-D bins (Nmodes, Nmodes_2D): every mode by the exact FP64 rules (mu has the sign of its frequency).
+// Also without them for more bins than k_mode_counts holds in shared memory.
+__global__ void __launch_bounds__(256) k_mode_counts_each(BinParams bp, BinTables t, unsigned long long *nm,
+                                                          unsigned long long *nm2d) {
   extern __shared__ unsigned long long scount[];
   const int nk = bp.nk, n2 = bp.out2d ? nk * bp.nmu : 0;
   for (int c = threadIdx.x; c < nk + n2; c += blockDim.x) scount[c] = 0;
@@ -269,6 +271,76 @@ __global__ void __launch_bounds__(256) k_mode_counts(BinParams bp, BinTables t, 
     if (c < nk) atomicAdd(nm + c, v);
     else atomicAdd(nm2d + (c - nk), v);
   }
+}
+
+// Mode counts without 2-D bins. s and the multiplicity are the same for ky and -ky, and s for kx and -kx, so a warp takes
+// a column (ky >= 0, kz) and its lanes 32 consecutive kx >= 0 at a time, each for all its signs, up to the top
+// edge. Along kx the bin is monotone: a run of lanes of one bin is one addition. The bin comes from FP32 s and the safe
+// edges, and from the exact FP64 s within a few ulps of an edge.
+// What bounds it: issue and, below 256^3, latency. Every mode in FP64 with an addition of its own took 44, 240 and 410 us at
+// 128^3, 192^3 and 256^3 (two fifths of a
+// batch of small boxes, which counts for each box); this takes 6, 9 and 13 us.
+__global__ void __launch_bounds__(256) k_mode_counts(BinParams bp, BinTables t, unsigned long long *nm) {
+  extern __shared__ unsigned long long scount[];
+  const int nk = bp.nk;
+  double *sE = (double *)(scount + nk);
+  float *sElo = (float *)(sE + nk + 3), *sEhi = sElo + nk + 3;
+  for (int c = threadIdx.x; c < nk; c += blockDim.x) scount[c] = 0;
+  for (int c = threadIdx.x; c < nk + 3; c += blockDim.x) {
+    sE[c] = t.E[c];
+    sElo[c] = t.Elo[c];
+    sEhi[c] = t.Ehi[c];
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, nkz = bp.kzmax + 1;
+  const long long ncol = (long long)(bp.ny / 2 + 1) * nkz, nw = (long long)gridDim.x * (blockDim.x / 32);
+  for (long long col = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; col < ncol; col += nw) {
+    const int j = (int)(col / nkz), k = (int)(col - (long long)j * nkz);
+    const int wy = j != 0 && 2 * j != bp.ny ? 2 : 1;
+    const float syz = t.fy2f[j] + t.fz2f[k];
+    const long long inner = 2 * wy * (k != 0 ? 2 : 1);  // a kx and its mirror, neither of them special
+    for (int i0 = 0; i0 <= bp.nx / 2; i0 += 32) {
+      const int i = i0 + lane;
+      int b = nk;
+      if (i <= bp.nx / 2) {
+        const float s = t.fx2f[i] + syz;
+        if (!bp.lg) {
+          const float v = (s > 0.0f ? s * rsqrtf(s) : 0.0f) * bp.kscale + bp.koff;
+          b = v < 0.0f ? -1 : (v >= (float)nk ? nk : (int)v);
+        } else {
+          int a = 0, z = nk + 2;  // sElo[a] <= s < sElo[z]
+          while (z - a > 1) {
+            const int mid = (a + z) >> 1;
+            if (sElo[mid] <= s) a = mid;
+            else z = mid;
+          }
+          b = a - 1;
+        }
+        while (b < nk && s >= sElo[b + 2]) b++;
+        while (b > -1 && s < sEhi[b + 1]) b--;
+        if (!(s >= sElo[b + 1] && s < sEhi[b + 2])) b = exact_bin(sE, nk, exact_s(t, i, j, k), b);
+      }
+      const int prev = __shfl_up_sync(0xffffffffu, b, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || b != prev);
+      if (b >= 0 && b < nk) {
+        long long add = 0;
+        if ((heads >> lane) & 1u) {
+          const unsigned later = lane == 31 ? 0u : heads >> (lane + 1);
+          add = inner * (later ? __ffs(later) : 32 - lane);
+        }
+        if (i == 0 || i >= bp.nx / 2 - 1 || i == bp.xhalf) {  // what this kx really counts
+          long long w = herm_nm(i, j, k, bp.xhalf);
+          if (i != 0 && 2 * i != bp.nx) w += herm_nm(bp.nx - i, j, k, bp.xhalf);
+          add += w * wy - inner;
+        }
+        if (add) atomicAdd(&scount[b], (unsigned long long)add);
+      }
+      if (__shfl_sync(0xffffffffu, b, 31) >= nk) break;
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < nk; c += blockDim.x)
+    if (scount[c]) atomicAdd(nm + c, scount[c]);
 }
 
 template <typename R>
@@ -1771,9 +1843,16 @@ void bin_params_kguess(BinParams &bp, const capow_params &p) {
 
 void launch_mode_counts(cudaStream_t s, const BinParams &bp, const BinTables &t, unsigned long long *nmodes,
                         unsigned long long *nmodes2d, long long *launches) {
-  const size_t smem = sizeof(unsigned long long) * (bp.nk + (bp.out2d ? bp.nk * bp.nmu : 0));
-  cudaFuncSetAttribute(k_mode_counts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_mode_counts<<<152 * 4, 256, smem, s>>>(bp, t, nmodes, nmodes2d);
+  const size_t smem = 8u * (size_t)bp.nk + 16u * (size_t)(bp.nk + 3);
+  if (bp.out2d || smem > 200 * 1024) {
+    const size_t each = sizeof(unsigned long long) * (bp.nk + (bp.out2d ? bp.nk * bp.nmu : 0));
+    cudaFuncSetAttribute(k_mode_counts_each, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each);
+    k_mode_counts_each<<<152 * 4, 256, each, s>>>(bp, t, nmodes, nmodes2d);
+  } else {
+    cudaFuncSetAttribute(k_mode_counts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const long long ncol = (long long)(bp.ny / 2 + 1) * (bp.kzmax + 1);  // a column per warp at least
+    k_mode_counts<<<(unsigned)std::min<long long>(152 * 4, (ncol + 7) / 8), 256, smem, s>>>(bp, t, nmodes);
+  }
   (*launches)++;
 }
 

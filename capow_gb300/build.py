@@ -22,7 +22,7 @@ BIN = os.path.join(HERE, "bin")
 LIB = os.path.join(BUILD, "libcapow_gpu.so")
 DRIVER = os.path.join(BIN, "capow")
 
-CU_SOURCES = ["capow_api.cu", "paint.cu", "bin.cu", "xbin.cu", "xrow_f2i.cu", "xrow_f1i.cu", "xrow_plain.cu", "noalloc.cu", "adjoint.cu", "batch.cu", "survey.cu"]
+CU_SOURCES = ["capow_api.cu", "paint.cu", "bin.cu", "xbin.cu", "xrow_f2i.cu", "xrow_f1i.cu", "xrow_plain.cu", "xsurvey.cu", "noalloc.cu", "adjoint.cu", "batch.cu", "survey.cu"]
 C_SOURCES = ["params.c", "catalogue.c", "output.c", "survey_io.c"]
 DRIVER_SOURCES = ["main.c"]
 

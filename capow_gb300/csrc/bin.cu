@@ -277,9 +277,9 @@ __global__ void __launch_bounds__(256) k_mode_counts_each(BinParams bp, BinTable
 // a column (ky >= 0, kz) and its lanes 32 consecutive kx >= 0 at a time, each for all its signs, up to the top
 // edge. Along kx the bin is monotone: a run of lanes of one bin is one addition. The bin comes from FP32 s and the safe
 // edges, and from the exact FP64 s within a few ulps of an edge.
-// What bounds it: issue and, below 256^3, latency. Every mode in FP64 with an addition of its own took 44, 240 and 410 us at
-// 128^3, 192^3 and 256^3 (two fifths of a
-// batch of small boxes, which counts for each box); this takes 6, 9 and 13 us.
+// What bounds it: issue and, below 256^3, latency. Every mode in FP64 with an addition of its own took 44, 240 and
+// 410 us at 128^3, 192^3 and 256^3 (two fifths of a batch of small boxes, which counts for each box); this takes 6, 9
+// and 13 us.
 __global__ void __launch_bounds__(256) k_mode_counts(BinParams bp, BinTables t, unsigned long long *nm) {
   extern __shared__ unsigned long long scount[];
   const int nk = bp.nk;

@@ -146,6 +146,22 @@ void launch_yfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int ns
                  const float2 *in, long long in_slot, float2 *out, long long out_slot);
 void launch_xrow(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg, void *const slots[4],
                  const double *dcv, double *bins, long long *launches);
+
+// The survey's fused x axis + assign pass on the same layout (xsurvey.cu). One FFT set:
+struct SvSet {
+  int l, m, xodd;       // h_lm (harm.cuh); xodd: it changes sign with kx (set by the launcher)
+  float coef;           // c_lm
+  float2 *F0, *F0m;     // monopole fields [kz][ky][NX]: the l = 0 set writes them, the others read
+  const double *dc;     // exact DC of each painted slot
+  int origin;           // the observer's cell (l = 0): painted grids, its index there, e^{-2 pi i q o/N} per axis
+  const float *a[4];
+  long long oind;
+  const float2 *ox, *oy, *oz;
+};
+bool xrow_geo(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg);  // blocks of either x pass
+bool xrow_survey_plan(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg);
+void launch_xrow_survey(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg, int nf, const float2 *u,
+                        long long uslot, SvSet set, double *bins);
 // DC corrections: dcv[slot] = painted sum (minus NGRID for mean-subtracted field A slots)
 void launch_dc_prepare(cudaStream_t s, const void *st, int deterministic, int nslot, int nfields, int mean_sub_a,
                        const double *fixed_scale, double *dcv, long long *launches);

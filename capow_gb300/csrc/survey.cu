@@ -659,6 +659,12 @@ struct capow_survey_ctx {
   bool tr;
   cufftHandle yplan, xplan;
   bool yplan_ok, xplan_ok;
+  // NX and NY powers of two as well: the blocked path, y by k_yfft into ubuf ([kz][ky][NX] per slot, rows below the
+  // top k-bin only), the x axis and the assign pass by k_xrow_survey; no cuFFT plan
+  bool blk;
+  float2 *ubuf;
+  long long uslot;
+  XbinGeo xg;
   // the observer's cell (r2 == 0), if any
   int origin;
   long long oind;
@@ -856,6 +862,17 @@ extern "C" int capow_survey_create(const capow_params *p, const capow_survey_par
   // FP32 with a power-of-two NZ: the transposed path (its z pass weights the painted grids as it reads
   // them, so no weighted grid is written; the y axis is then a contiguous batched transform)
   if (!f64 && c->bt.twz && zr2c_supported(bp)) {
+    if (xrow_survey_plan(bp, c->bt, c->nslot, c->xg)) {
+      void *ub = nullptr;
+      c->uslot = (long long)(bp.kzmax + 1) * p->NY * p->NX;
+      if (cudaMalloc(&ub, sizeof(float2) * (size_t)c->uslot * c->nslot) == cudaSuccess) {
+        c->allocs.push_back(ub);
+        c->ubuf = (float2 *)ub;
+        c->tr = c->blk = true;
+        return CAPOW_OK;
+      }
+      (void)cudaGetLastError();  // no room: the transforms in place below
+    }
     const long long yrows = (long long)c->nslot * p->NX * bp.nzc, xcols = (long long)bp.nzc * p->NY;
     int ny = p->NY, nx = p->NX, emb = p->NX;
     if (yrows <= 0x7fffffffLL && xcols <= 0x7fffffffLL &&
@@ -1100,6 +1117,19 @@ static int sv_multipoles(capow_survey_ctx *c) {
   sa.ox = (const C *)c->ox;
   sa.oy = (const C *)c->oy;
   sa.oz = (const C *)c->oz;
+  SvSet set;
+  memset(&set, 0, sizeof set);
+  if constexpr (sizeof(R) == 4) {
+    set.F0 = sa.F0;
+    set.F0m = sa.F0m;
+    set.dc = sa.dc;
+    set.origin = sa.origin;
+    for (int s = 0; s < 4; s++) set.a[s] = sa.a[s];
+    set.oind = sa.oind;
+    set.ox = sa.ox;
+    set.oy = sa.oy;
+    set.oz = sa.oz;
+  }
   const int step = p.Odd_Multipoles ? 1 : 2;  // src/main.c:490-492
   c->sets = 0;
   for (int l = 0; l <= 4; l += step) {
@@ -1115,6 +1145,16 @@ static int sv_multipoles(capow_survey_ctx *c) {
             launch_zr2c_weighted(c->stream, c->bp, c->bt, c->nslot, (const float *)a[0], ge, (int)g.row,
                                  (float2 *)w[0], tslot, (const float *)c->vx, (const float *)c->vy,
                                  (const float *)c->vz, l, m, &c->launches);
+          if (c->blk) {
+            launch_yfft(c->stream, c->bp, c->bt, c->nslot, 0, p.NX, (const float2 *)w[0], tslot, c->ubuf, c->uslot);
+            set.l = l;
+            set.m = m;
+            set.coef = (float)harm_coef(l, m);
+            launch_xrow_survey(c->stream, c->bp, c->bt, c->xg, nf, c->ubuf, c->uslot, set, c->bins);
+            c->launches++;
+            c->sets++;
+            continue;
+          }
           CKFFT(c, cufftExecC2C(c->yplan, (cufftComplex *)w[0], (cufftComplex *)w[0], CUFFT_FORWARD));
           for (int s = 0; s < c->nslot; s++)
             CKFFT(c, cufftExecC2C(c->xplan, (cufftComplex *)w[s], (cufftComplex *)w[s], CUFFT_FORWARD));

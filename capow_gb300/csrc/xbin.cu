@@ -131,7 +131,7 @@ void launch_yfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int ns
 }
 
 // ---------------------------------------------------------------------------------- x axis + binning
-bool xrow_plan(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg) {
+bool xrow_geo(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg) {
   const int n = bp.nx;
   if (n < 64 || n > 1024 || (n & (n - 1)) != 0 || bp.out2d || !yfft_supported(bp, t) || nslot == 3) return false;
   memset(&xg, 0, sizeof xg);
@@ -146,6 +146,11 @@ bool xrow_plan(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg) 
   xg.n_inner = bp.ny;
   xg.nkb = bp.ny >> xg.log2kc;
   xg.nblocks = xg.n_outer * xg.nkb;
+  return true;
+}
+
+bool xrow_plan(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg) {
+  if (!xrow_geo(bp, t, nslot, xg)) return false;
   const int np = xrow_products(bp), nl = xrow_multipoles(bp);
   // two copies of the block bins while two CTAs fit an SM, else one
   xg.nbc = 2;

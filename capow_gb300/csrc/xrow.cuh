@@ -89,6 +89,94 @@ __device__ __forceinline__ void xr_columns(const float2 *g0, const float2 *g1, c
   __syncthreads();
 }
 
+// The k-bin of the mode (i, column) with |f|^2 = s (src/main.c:355, 369-375); nk beyond the column's last |kx|. sE,
+// sElo, sEhi: the edges in shared memory.
+__device__ __forceinline__ int xr_mode_bin(const BinParams &bp, const BinTables &t, const double *sE, const float *sElo,
+                                           const float *sEhi, const XrCol &col, int i, float s) {
+  const int nk = bp.nk;
+  int b = nk;
+  if (i <= col.r) {
+    if (!bp.lg) {
+      const float v = (s > 0.0f ? s * rsqrtf(s) : 0.0f) * bp.kscale + bp.koff;
+      b = v < 0.0f ? -1 : (v >= (float)nk ? nk : (int)v);
+    } else {
+      int a = 0, z = nk + 2;  // sElo[a] <= s < sElo[z]
+      while (z - a > 1) {
+        const int mid = (a + z) >> 1;
+        if (sElo[mid] <= s) a = mid;
+        else z = mid;
+      }
+      b = a - 1;
+    }
+    while (b < nk && s >= sElo[b + 2]) b++;
+    while (b > -1 && s < sEhi[b + 1]) b--;
+    if (!(s >= sElo[b + 1] && s < sEhi[b + 2]))  // within a few ulps of an edge: the exact FP64 s decides
+      b = exact_bin(sE, nk, __dadd_rn(__dadd_rn(t.fx2d[i], t.fy2d[col.j]), t.fz2d[col.kz]), b);
+  }
+  return b;
+}
+
+// Add each lane's NA sums to row q of dst ([NA][nk]) at its bin b (in: b is a bin; lanes of one bin are a run): the sum of
+// a run is gathered to its first lane, which adds it.
+template <int NA>
+__device__ __forceinline__ void xr_add_runs(float (&acc)[NA], int b, bool in, int lane, float *dst, int nk) {
+  const int prev = __shfl_up_sync(FULL_MASK, b, 1);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int b2 = __shfl_down_sync(FULL_MASK, b, o);
+    const bool same = lane + o < 32 && b2 == b;
+    if (!__any_sync(FULL_MASK, same && in)) break;
+#pragma unroll
+    for (int q = 0; q < NA; q++) {
+      const float v = __shfl_down_sync(FULL_MASK, acc[q], o);
+      if (same) acc[q] += v;
+    }
+  }
+  if (in && (lane == 0 || prev != b)) {
+#pragma unroll
+    for (int q = 0; q < NA; q++) atomicAdd(&dst[q * nk + b], acc[q]);
+  }
+}
+
+// First block at or after blk (in steps of the grid) that reaches below the top edge: fz^2 grows with kz; fy^2 rises to
+// ky = NY/2 and falls after it, so over a run of KC ky it is smallest at an end.
+template <int KC>
+__device__ __forceinline__ int xr_next_live(const BinTables &t, const XbinGeo &xg, float top, int blk) {
+  for (; blk < xg.nblocks; blk += gridDim.x) {
+    const int kz = blk / xg.nkb, j0 = (blk - kz * xg.nkb) * KC;
+    if (!(t.fz2f[kz] + fminf(t.fy2f[j0], t.fy2f[j0 + KC - 1]) > top)) break;
+  }
+  return blk;
+}
+
+// The kx-independent quantities of the column (ky j, kz) (src/main.c:335-389 for the y, z factors).
+template <bool IL>
+__device__ __forceinline__ XrCol xr_column(const BinParams &bp, const BinTables &t, int j, int kz, float top, float inv_fx) {
+  XrCol col;
+  col.syz = t.fy2f[j] + t.fz2f[kz];
+  float cyz = t.cyf[j] * t.czf[kz];
+  if (IL) cyz *= 0.25f;
+  col.cyzn = kz != 0 ? 2.0f * cyz : cyz;  // Hermitian multiplicity off the kz = 0 plane (:422-429)
+  col.eyz = IL ? cmulf(t.eyf[j], t.ezf[kz]) : make_float2(0.0f, 0.0f);
+  col.flos = bp.los == 2 ? t.fyf[j] : t.fzf[kz];
+  col.j = j;
+  col.kz = kz;
+  const float rest = top - col.syz;
+  col.r = rest > 0.0f ? min(bp.nx / 2, (int)(sqrtf(rest) * inv_fx) + 1) : -1;
+  return col;
+}
+
+// FP32 block bins (nbc copies) to the CTA's FP64 bins.
+__device__ __forceinline__ void xr_flush(float *sb, double *sbd, int nbins, int nbc) {
+  for (int c = threadIdx.x; c < nbins; c += blockDim.x) {
+    float v = 0.0f;
+    for (int k = 0; k < nbc; k++) {
+      v += sb[c + k * nbins];
+      sb[c + k * nbins] = 0.0f;
+    }
+    sbd[c] += (double)v;
+  }
+}
+
 // The fused pass. Blocks of kc columns of every slot (16 columns of 512 values: 64 KB, two CTAs per SM, so that one
 // computes while the other waits for its block, whose lines an L2 prefetch of contiguous runs has brought near).
 //
@@ -148,47 +236,23 @@ __global__ void __launch_bounds__(xr_threads(LN), 2)
   const float topf32 = (float)t.E[nk + 1] * 1.0001f;
   const float inv_fx = 1.0f / bp.fx_step;
   const long long blk_elems = (long long)N * KC;
-  // first block at or after blk (in steps of the grid) that reaches below the top edge: fz^2 grows with kz; fy^2
-  // rises to ky = NY/2 and falls after it, so over a run of ky it is smallest at an end
-  auto next_live = [&](int blk) {
-    for (; blk < xg.nblocks; blk += gridDim.x) {
-      const int kz = blk / xg.nkb, j0 = (blk - kz * xg.nkb) * KC;
-      if (!(t.fz2f[kz] + fminf(t.fy2f[j0], t.fy2f[j0 + KC - 1]) > topf32)) break;
-    }
-    return blk;
-  };
   float *sbw = sb + (warp & (xg.nbc - 1)) * nbins;  // this warp's copy
   int nproc = 0;
-  if (threadIdx.x == 0) s_next = next_live(blockIdx.x);
+  if (threadIdx.x == 0) s_next = xr_next_live<KC>(t, xg, topf32, blockIdx.x);
   __syncthreads();
   int blk = s_next;
   __syncthreads();  // s_next is read before the loop writes it again
   while (blk < xg.nblocks) {
     const int kz = blk / xg.nkb, j0 = (blk - kz * xg.nkb) * KC;
     if (warp == XR_THREADS / 32 - 1) {  // the next block (read after the barriers below), and its runs towards L2
-      const int nxt = next_live(blk + gridDim.x);
+      const int nxt = xr_next_live<KC>(t, xg, topf32, blk + gridDim.x);
       if (lane == 0) s_next = nxt;
       if (lane < NS && nxt < xg.nblocks) {
         const float2 *q = (lane == 0 ? g0 : (lane == 1 ? g1 : (lane == 2 ? g2 : g3))) + (long long)nxt * blk_elems;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(q), "r"((unsigned)(blk_elems * 8)) : "memory");
       }
     }
-    // the block's columns (src/main.c:335-389 for the y, z factors)
-    if (threadIdx.x < KC) {
-      XrCol col;
-      const int j = j0 + threadIdx.x;
-      col.syz = t.fy2f[j] + t.fz2f[kz];
-      float cyz = t.cyf[j] * t.czf[kz];
-      if (IL) cyz *= 0.25f;
-      col.cyzn = kz != 0 ? 2.0f * cyz : cyz;  // Hermitian multiplicity off the kz = 0 plane (:422-429)
-      col.eyz = IL ? cmulf(t.eyf[j], t.ezf[kz]) : make_float2(0.0f, 0.0f);
-      col.flos = bp.los == 2 ? t.fyf[j] : t.fzf[kz];
-      col.j = j;
-      col.kz = kz;
-      const float topf = sElo[nk + 1] - col.syz;
-      col.r = topf > 0.0f ? min(HALF, (int)(sqrtf(topf) * inv_fx) + 1) : -1;
-      scol[threadIdx.x] = col;
-    }
+    if (threadIdx.x < KC) scol[threadIdx.x] = xr_column<IL>(bp, t, j0 + threadIdx.x, kz, sElo[nk + 1], inv_fx);
     xr_columns<LN, NS>(g0, g1, g2, g3, (long long)blk * blk_elems, sd, stw);
     constexpr int NJ = (HALF + 32) / 32;  // warps' worth of kx = 0 .. NX/2
     for (int task = warp; task < KC * NJ; task += XR_THREADS / 32) {
@@ -196,31 +260,12 @@ __global__ void __launch_bounds__(xr_threads(LN), 2)
       const XrCol col = scol[c];
       if (i - lane > col.r) continue;
       const unsigned char *F0 = sd + c * COLB, *F1 = F0 + KC * COLB;
-      // ---- the bin of (i, column) (src/main.c:355, 369-375)
       const int ic = min(i, HALF);
       const float4 xt = sxt[ic];
       const float s = xt.x + col.syz;
-      int b = nk;
-      if (i <= col.r) {
-        if (!bp.lg) {
-          const float v = (s > 0.0f ? s * rsqrtf(s) : 0.0f) * bp.kscale + bp.koff;
-          b = v < 0.0f ? -1 : (v >= (float)nk ? nk : (int)v);
-        } else {
-          int a = 0, z = nk + 2;  // sElo[a] <= s < sElo[z]
-          while (z - a > 1) {
-            const int mid = (a + z) >> 1;
-            if (sElo[mid] <= s) a = mid;
-            else z = mid;
-          }
-          b = a - 1;
-        }
-        while (b < nk && s >= sElo[b + 2]) b++;
-        while (b > -1 && s < sEhi[b + 1]) b--;
-        if (!(s >= sElo[b + 1] && s < sEhi[b + 2]))  // within a few ulps of an edge: the exact FP64 s decides
-          b = exact_bin(sE, nk, __dadd_rn(__dadd_rn(t.fx2d[i], t.fy2d[col.j]), t.fz2d[col.kz]), b);
-      }
+      const int b = xr_mode_bin(bp, t, sE, sElo, sEhi, col, i, s);
       const bool in = b >= 0 && b < nk;
-      float acc[NPU][NL];
+      float acc[NPU * NL];
       {
         const bool pair = i != 0 && i != HALF;  // kx = 0 and NX/2 have no mirror
         float Pe[NPU], Po[NPU];  // products summed over the pair, and with the mirror's sign of mu
@@ -286,49 +331,21 @@ __global__ void __launch_bounds__(xr_threads(LN), 2)
 #pragma unroll
         for (int q = 0; q < NPU; q++) {
           const float p = in ? Pe[q] * gc : 0.0f;  // (columns beyond the top edge hold no values)
-          acc[q][0] = p;
-          acc[q][1] = p * L2;
-          acc[q][2] = p * L4;
+          acc[q * NL] = p;
+          acc[q * NL + 1] = p * L2;
+          acc[q * NL + 2] = p * L4;
           if (ODD) {
             const float o = in ? Po[q] * gc : 0.0f;
-            acc[q][NL - 2] = o * mu;
-            acc[q][NL - 1] = o * ((2.5f * mu2 - 1.5f) * mu);
+            acc[q * NL + NL - 2] = o * mu;
+            acc[q * NL + NL - 1] = o * ((2.5f * mu2 - 1.5f) * mu);
           }
         }
       }
-      // the sum of each run of lanes of one bin, at the run's first lane
-      const int prev = __shfl_up_sync(FULL_MASK, b, 1);
-      for (int o = 1; o < 32; o <<= 1) {
-        const int b2 = __shfl_down_sync(FULL_MASK, b, o);
-        const bool same = lane + o < 32 && b2 == b;
-        if (!__any_sync(FULL_MASK, same && in)) break;
-#pragma unroll
-        for (int q = 0; q < NPU; q++)
-#pragma unroll
-          for (int l = 0; l < NL; l++) {
-            const float v = __shfl_down_sync(FULL_MASK, acc[q][l], o);
-            if (same) acc[q][l] += v;
-          }
-      }
-      if (in && (lane == 0 || prev != b)) {
-#pragma unroll
-        for (int q = 0; q < NPU; q++)
-#pragma unroll
-          for (int l = 0; l < NL; l++) atomicAdd(&sbw[(q * NL + l) * nk + b], acc[q][l]);
-      }
+      xr_add_runs<NPU * NL>(acc, b, in, lane, sbw, nk);
     }
     blk = s_next;
-    __syncthreads();  // the binning has read sd, scol and sedge
-    if ((++nproc & 15) == 0) {
-      for (int c = threadIdx.x; c < nbins; c += XR_THREADS) {
-        float v = 0.0f;
-        for (int k = 0; k < xg.nbc; k++) {
-          v += sb[c + k * nbins];
-          sb[c + k * nbins] = 0.0f;
-        }
-        sbd[c] += (double)v;
-      }
-    }
+    __syncthreads();  // the binning has read sd and scol
+    if ((++nproc & 15) == 0) xr_flush(sb, sbd, nbins, xg.nbc);
   }
   __syncthreads();
   // CTA bins (FP64) -> global FP64 bins [product][5][nk]; stored product and multipole index -> q, l

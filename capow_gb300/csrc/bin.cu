@@ -634,6 +634,179 @@ __global__ void __launch_bounds__(256) k_bin(BinParams bp, BinTables t, const ty
     }
 }
 
+// The FP64 bin kernel without 2-D bins. A thread takes the columns (ky, kz) and (-ky, kz) and walks kx >= 0, each step for
+// kx and -kx: up to four modes that share s, the bin, the weights and the Legendre factors. (i, j) and their mirrors keep
+// the sums of k_bin; mu^2 = f^2 / s needs no square root when no odd multipole is asked for.
+// What bounds it: the FP64 pipe (71% busy). 256^3, two fields, interlaced, three spectra: 0.55 ms, 1.51 by k_bin<double> (a
+// mode at a time, with a square root and a division each).
+template <int NF, bool ODD>
+__global__ void __launch_bounds__(256) k_bin64(BinParams bp, BinTables t, const double2 *gA, const double2 *gB,
+                                               const double2 *gAi, const double2 *gBi, const double *dcv, double *bins,
+                                               int ichunk) {
+  constexpr int NP = NF == 1 ? 1 : 4;
+  const int nk = bp.nk;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const BinSmem L = bin_smem_layout(8, NP, nk, 0, ichunk);
+  double *sb = (double *)(smraw + L.sb);
+  double *sE = (double *)(smraw + L.sE);
+  float *sElo = (float *)(smraw + L.sElo);
+  double *sfx2 = (double *)(smraw + L.sfx2);
+  double *scx = (double *)(smraw + L.scx);
+  double2 *sex = (double2 *)(smraw + L.sex);
+  double *sfl = (double *)(smraw + L.sfl);
+  const int i0 = blockIdx.y * ichunk, i1 = min(bp.nx / 2 + 1, i0 + ichunk);
+  for (int c = threadIdx.x; c < NP * 5 * nk; c += blockDim.x) sb[c] = 0.0;
+  for (int c = threadIdx.x; c < nk + 3; c += blockDim.x) {
+    sE[c] = t.E[c];
+    sElo[c] = t.Elo[c];
+  }
+  for (int c = threadIdx.x; c < i1 - i0; c += blockDim.x) {
+    sfx2[c] = t.fx2d[i0 + c];
+    scx[c] = t.cxd[i0 + c];
+    sex[c] = t.exd[i0 + c];
+    sfl[c] = t.fxd[i0 + c];
+  }
+  __syncthreads();
+  const long long cols = (long long)bp.ny * bp.nzc;
+  const long long col = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int j = (int)(col / bp.nzc), k = (int)(col - (long long)j * bp.nzc);
+  if (j <= bp.ny / 2) {
+    const int nj = j != 0 && 2 * j != bp.ny ? 2 : 1;
+    const double fy2 = t.fy2d[j], fz2 = t.fz2d[k];
+    double cyz = t.cyd[j] * t.czd[k];
+    if (bp.interlace) cyz *= 0.25;
+    if (k != 0) cyz *= 2.0;  // Hermitian multiplicity off the kz = 0 plane
+    double2 eyz[2];          // of ky and -ky
+    {
+      const double2 a = t.eyd[j], b = t.ezd[k];
+      eyz[0] = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+      eyz[1] = make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
+    }
+    const double flos = bp.los == 2 ? t.fyd[j] : t.fzd[k];
+    double acc[NP][5];
+#pragma unroll
+    for (int q = 0; q < NP; q++)
+#pragma unroll
+      for (int l = 0; l < 5; l++) acc[q][l] = 0.0;
+    const float top = sElo[nk + 1] - (float)(fy2 + fz2);
+    const int r = top > 0.0f ? min(bp.nx / 2, (int)(sqrtf(top) / bp.fx_step) + 1) : -1;
+    int cur = -1;
+    double hi = -1.0;  // upper edge of the current bin (before the first step: search)
+    auto flush = [&]() {
+      if (cur >= 0 && cur < nk) {
+#pragma unroll
+        for (int q = 0; q < NP; q++)
+#pragma unroll
+          for (int l = 0; l < 5; l++) {
+            if ((l == 1 || l == 3) && !ODD) continue;
+            if (acc[q][l] != 0.0) atomicAdd(&sb[(q * 5 + l) * nk + cur], acc[q][l]);
+            acc[q][l] = 0.0;
+          }
+      }
+    };
+    for (int i = i0; i < i1 && i <= r; i++) {
+      const int li = i - i0;
+      const double s = __dadd_rn(__dadd_rn(sfx2[li], fy2), fz2);  // rises with i
+      if (!(s < hi)) {
+        int b = cur;
+        if (hi < 0.0 && !bp.lg) b = (int)fminf(sqrtf((float)s) * bp.kscale + bp.koff, (float)nk);
+        b = exact_bin(sE, nk, s, b);
+        hi = sE[b + 2];
+        if (b != cur) flush();
+        cur = b;
+        if (cur >= nk) break;
+      }
+      if (cur < 0) continue;
+      double Pe[NP], Po[NP];  // the modes' products, and with the sign of mu
+#pragma unroll
+      for (int q = 0; q < NP; q++) Pe[q] = Po[q] = 0.0;
+      const double2 ex = sex[li];
+#pragma unroll
+      for (int mj = 0; mj < 2; mj++) {
+        if (mj >= nj) break;
+        const long long base = (long long)(mj ? bp.ny - j : j) * bp.nzc + k;
+#pragma unroll
+        for (int mi = 0; mi < 2; mi++) {
+          if (mi && (i == 0 || 2 * i == bp.nx)) break;
+          const int ii = mi ? bp.nx - i : i;
+          const long long off = ii * cols + base;
+          const bool dc = ii == 0 && base == 0;
+          double2 A = gA[off], B = make_double2(0.0, 0.0);
+          if (NF == 2) B = gB[off];
+          if (dc) {  // the slots' exact DC values replace F(0)
+            A = make_double2(dcv[0], 0.0);
+            if (NF == 2) B = make_double2(dcv[1], 0.0);
+          }
+          if (bp.interlace) {
+            const double exy = mi ? -ex.y : ex.y;
+            const double2 e = make_double2(ex.x * eyz[mj].x - exy * eyz[mj].y, ex.x * eyz[mj].y + exy * eyz[mj].x);
+            double2 a = gAi[off];
+            if (dc) a = make_double2(dcv[NF], 0.0);
+            A.x += a.x * e.x - a.y * e.y;
+            A.y += a.x * e.y + a.y * e.x;
+            if (NF == 2) {
+              double2 b2 = gBi[off];
+              if (dc) b2 = make_double2(dcv[3], 0.0);
+              B.x += b2.x * e.x - b2.y * e.y;
+              B.y += b2.x * e.y + b2.y * e.x;
+            }
+          }
+          const bool neg = (bp.los == 1 && mi) || (bp.los == 2 && mj);
+          auto add = [&](int q, double ax, double bx, double ay, double by) {  // Pe += ax bx + ay by
+            if (!(bp.pmask & (1 << q))) return;  // a product no requested spectrum reads
+            if (ODD) {
+              const double p = ax * bx + ay * by;
+              Pe[q] += p;
+              Po[q] += neg ? -p : p;
+            } else {
+              Pe[q] = fma(ax, bx, fma(ay, by, Pe[q]));
+            }
+          };
+          // NM on the kz = 0 plane (src/main.c:422-429): a mode that counts twice is added twice
+          const int reps = k == 0 ? herm_nm(ii, mj ? bp.ny - j : j, 0, bp.xhalf) : 1;
+          for (int rep = 0; rep < reps; rep++) {
+            add(0, A.x, A.x, A.y, A.y);
+            if (NF == 2) {
+              add(1, A.x, B.x, A.y, B.y);
+              add(2, A.x, B.y, -A.y, B.x);
+              add(3, B.x, B.x, B.y, B.y);
+            }
+          }
+        }
+      }
+      const double gc = cyz * scx[li];
+      const double fl = bp.los == 1 ? sfl[li] : flos;
+      double mu = 0.0, mu2 = 0.0;
+      if (ODD) {
+        mu = s > 0.0 ? fl / sqrt(s) : 0.0;
+        mu2 = mu * mu;
+      } else {
+        mu2 = s > 0.0 ? fl * fl / s : 0.0;
+      }
+      const double L2 = 1.5 * mu2 - 0.5;
+      const double L4 = (4.375 * mu2 - 3.75) * mu2 + 0.375;
+#pragma unroll
+      for (int q = 0; q < NP; q++) {
+        if (!(bp.pmask & (1 << q))) continue;
+        const double p = Pe[q] * gc;
+        acc[q][0] += p;
+        acc[q][2] += p * L2;
+        acc[q][4] += p * L4;
+        if (ODD) {
+          const double o = Po[q] * gc * mu;
+          acc[q][1] += o;
+          acc[q][3] += o * (2.5 * mu2 - 1.5);
+        }
+      }
+    }
+    flush();
+  }
+  __syncthreads();
+  // CTA bins -> global bins, laid out [product][5][nk]
+  for (int c = threadIdx.x; c < NP * 5 * nk; c += blockDim.x)
+    if (sb[c] != 0.0) atomicAdd(&bins[c], sb[c]);
+}
+
 // ------------------------------------------------------------ fused x-axis FFT + binning (FP32)
 // Every x-plane of every grid has been transformed over (y, z) (by cuFFT in place, or by k_zr2c and
 // the y-axis C2C into the transposed layout); what is left of the 3-D transform (src/main.c:266-271)
@@ -1890,14 +2063,33 @@ static void launch_bin_t(cudaStream_t s, const BinParams &bp, const BinTables &t
                                                                 sm2d);
 }
 
+template <int NF, bool ODD>
+static void launch_bin64(cudaStream_t s, const BinParams &bp, const BinTables &t, void *const slots[4], const double *dcv,
+                         double *bins) {
+  const long long cols = (long long)(bp.ny / 2 + 1) * bp.nzc;
+  const int half = bp.nx / 2 + 1, nbx = (int)((cols + 255) / 256);
+  // about four resident waves of two CTAs: columns near the top edge are short
+  int nchunk = std::min(half, std::max(1, (152 * 8 + nbx - 1) / nbx));
+  const int ichunk = (half + nchunk - 1) / nchunk;
+  nchunk = (half + ichunk - 1) / ichunk;
+  const size_t smem = bin_smem_layout(8, NF == 1 ? 1 : 4, bp.nk, 0, ichunk).total;
+  cudaFuncSetAttribute(k_bin64<NF, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const bool il = bp.interlace != 0;
+  k_bin64<NF, ODD><<<dim3(nbx, nchunk), 256, smem, s>>>(
+      bp, t, (const double2 *)slots[0], NF == 2 ? (const double2 *)slots[1] : nullptr,
+      il ? (const double2 *)slots[NF] : nullptr, il && NF == 2 ? (const double2 *)slots[NF + 1] : nullptr, dcv, bins, ichunk);
+}
+
 template <typename R, int NF>
 static void launch_bin_r(cudaStream_t s, const BinParams &bp, const BinTables &t, void *const slots[4],
                          const double *dcv, double *bins, double *bins2d) {
   if (bp.odd) {
     if (bp.out2d) launch_bin_t<R, NF, true, true>(s, bp, t, slots, dcv, bins, bins2d);
+    else if constexpr (sizeof(R) == 8) launch_bin64<NF, true>(s, bp, t, slots, dcv, bins);
     else launch_bin_t<R, NF, true, false>(s, bp, t, slots, dcv, bins, bins2d);
   } else {
     if (bp.out2d) launch_bin_t<R, NF, false, true>(s, bp, t, slots, dcv, bins, bins2d);
+    else if constexpr (sizeof(R) == 8) launch_bin64<NF, false>(s, bp, t, slots, dcv, bins);
     else launch_bin_t<R, NF, false, false>(s, bp, t, slots, dcv, bins, bins2d);
   }
 }

@@ -762,7 +762,6 @@ struct BucketOut {
 // on the same addresses: 2,097,152 such particles took 337 us into the 256 tiles of a 128^3 grid when each run
 // of lanes made its own.
 constexpr int BK_THREADS = 512;
-constexpr int BK_DIRECT_TILES = 4096;  // 16 KB of counters
 constexpr int BK_PPT = 4;              // particles per thread and chunk, at most
 constexpr int BK_P = BK_THREADS * BK_PPT;
 constexpr int BK_E = 4096;             // entries held; any beyond go out one by one

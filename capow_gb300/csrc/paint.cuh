@@ -68,6 +68,9 @@ struct PaintBufs {
   const cudaEvent_t *chunk_ev;
 };
 
+// Grids of up to this many tiles are bucketed by k_bucket_cta (16 KB of counters), larger ones by k_bucket_warp.
+constexpr int BK_DIRECT_TILES = 4096;
+
 // host launchers (paint.cu)
 void launch_paint64(cudaStream_t s, const Geom &g, const FieldSpec &fs, int dtype, const void *x, const void *y,
                     const void *z, const void *v, const void *w, long long n, const GridPtrs &grids, DevStats *st,

@@ -23,7 +23,11 @@ CASES = [
     # few and dense tiles: one CTA, clusters, two limbs
     ((32, 32, 32), 5000, 3, 3, 0, 1), ((32, 32, 32), 400000, 2, 0, 1, 1), ((16, 32, 32), 300000, 3, 0, 0, 0),
     ((33, 17, 65), 250000, 3, 2, 0, 1), ((8, 8, 8), 200000, 2, 0, 0, 1), ((64, 64, 64), 900000, 2, 0, 1, 0),
-    ((4, 300, 4), 150000, 3, 1, 0, 1), ((64, 64, 64), 2000000, 3, 3, 0, 1)]
+    ((4, 300, 4), 150000, 3, 1, 0, 1), ((64, 64, 64), 2000000, 3, 3, 0, 1),
+    # tiles away from the grid's faces: every order, periodic and not, one and two fields
+    ((64, 64, 128), 200000, 3, 0, 1, 1), ((64, 64, 128), 200000, 3, 2, 0, 0), ((64, 64, 128), 200000, 2, 0, 0, 1),
+    ((64, 64, 128), 200000, 2, 3, 0, 1), ((64, 64, 128), 200000, 2, 0, 1, 1), ((64, 64, 128), 50000, 1, 0, 1, 1),
+    ((40, 60, 112), 1000, 3, 3, 0, 1)]
 
 
 @pytest.mark.parametrize("shape,n,order,los,mom,il", CASES)

@@ -133,7 +133,7 @@ void launch_yfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int ns
 // ---------------------------------------------------------------------------------- x axis + binning
 bool xrow_geo(const BinParams &bp, const BinTables &t, int nslot, XbinGeo &xg) {
   const int n = bp.nx;
-  if (n < 64 || n > 1024 || (n & (n - 1)) != 0 || bp.out2d || !yfft_supported(bp, t) || nslot == 3) return false;
+  if (n < 32 || n > 1024 || (n & (n - 1)) != 0 || bp.out2d || !yfft_supported(bp, t) || nslot == 3) return false;
   memset(&xg, 0, sizeof xg);
   while ((1 << xg.log2n) < n) xg.log2n++;
   xg.ncol = xr_threads(xg.log2n) / (int)xr_lanes(xg.log2n);

@@ -23,9 +23,10 @@ CAPOW_HD constexpr unsigned xr_align(unsigned x) { return (x + 15u) & ~15u; }
 CAPOW_HD constexpr unsigned xr_col_bytes(int log2n, int ns) { return (ns == 1 ? 8u : 16u) * (1u << log2n) + 16u; }
 
 // Values of the row buffer that RowFft exchanges through, and lanes per row (fft_dev.cuh).
-CAPOW_HD constexpr unsigned xr_lanes(int log2n) { return log2n >= 9 ? 32u : (log2n == 8 ? 16u : 8u); }
-// Threads of a CTA (two CTAs per SM): 64 registers a thread for 8 or 16 values, 128 for the 32 of NX = 1024.
-CAPOW_HD constexpr int xr_threads(int log2n) { return log2n == 10 ? 256 : 512; }
+CAPOW_HD constexpr unsigned xr_lanes(int log2n) { return log2n >= 9 ? 32u : (log2n == 8 ? 16u : (log2n == 5 ? 4u : 8u)); }
+// Threads of a CTA (two CTAs per SM): 64 registers a thread for 8 or 16 values, 128 for the 32 of NX = 1024; half as
+// many for NX = 32, whose grids have few blocks.
+CAPOW_HD constexpr int xr_threads(int log2n) { return log2n == 10 || log2n == 5 ? 256 : 512; }
 CAPOW_HD constexpr unsigned xr_rowbuf(int log2n) { return ((1u << log2n) / xr_lanes(log2n)) * (xr_lanes(log2n) + 1u); }
 
 // Per-column quantities of the block being binned: everything of a mode that does not depend on kx.
@@ -380,6 +381,7 @@ template <int NF, bool IL, bool ODD, int PM>
 static void launch_xrow_t(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg,
                           void *const slots[4], const double *dcv, double *bins) {
   switch (xg.log2n) {
+    case 5: return launch_xrow_n<NF, IL, ODD, PM, 5>(s, bp, t, xg, slots, dcv, bins);
     case 6: return launch_xrow_n<NF, IL, ODD, PM, 6>(s, bp, t, xg, slots, dcv, bins);
     case 7: return launch_xrow_n<NF, IL, ODD, PM, 7>(s, bp, t, xg, slots, dcv, bins);
     case 8: return launch_xrow_n<NF, IL, ODD, PM, 8>(s, bp, t, xg, slots, dcv, bins);

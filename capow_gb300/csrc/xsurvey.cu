@@ -208,6 +208,8 @@ template <int NF, bool IL>
 static void launch_xs_t(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg, const float2 *u,
                         long long uslot, const SvSet &set, double *bins) {
   switch (xg.log2n * 2 + (set.l == 0)) {
+    case 10: return launch_xs_n<NF, IL, false, 5>(s, bp, t, xg, u, uslot, set, bins);
+    case 11: return launch_xs_n<NF, IL, true, 5>(s, bp, t, xg, u, uslot, set, bins);
     case 12: return launch_xs_n<NF, IL, false, 6>(s, bp, t, xg, u, uslot, set, bins);
     case 13: return launch_xs_n<NF, IL, true, 6>(s, bp, t, xg, u, uslot, set, bins);
     case 14: return launch_xs_n<NF, IL, false, 7>(s, bp, t, xg, u, uslot, set, bins);

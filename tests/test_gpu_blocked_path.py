@@ -1,4 +1,4 @@
-"""Power-of-two NX (64 to 1024), NY and NZ: z by k_zfft, y by k_yfft, the x axis and the binning by k_xrow_bin.
+"""Power-of-two NX (32 to 1024), NY and NZ: z by k_zfft, y by k_yfft, the x axis and the binning by k_xrow_bin.
 Held to the oracle and to the 3-D cuFFT + k_bin path on the same catalogue, at the suite's FP32 tolerances, over
 every row length of the three kernels, one to four slots, even and odd multipoles, linear and logarithmic bins from one
 bin to several hundred, the lines of sight, and top edges from beyond the Nyquist frequency (nothing left out) to a small
@@ -24,7 +24,9 @@ CASES = [((64, 16, 32), 3, 3, 1, 1, 1, dict(NK=24, Maxk=0.55)),
          ((1024, 32, 64), 3, 1, 1, 0, 0, dict(NK=64, Maxk=0.1)),
          ((1024, 16, 128), 2, 3, 1, 1, 1, dict(NK=20, Maxk=0.05)),
          ((64, 256, 1024), 2, 2, 0, 1, 0, dict(NK=12, Maxk=0.02)),
-         ((64, 512, 2048), 1, 0, 1, 0, 0, dict(NK=500, Maxk=0.2))]
+         ((64, 512, 2048), 1, 0, 1, 0, 0, dict(NK=500, Maxk=0.2)),
+         ((32, 32, 32), 3, 3, 1, 1, 1, dict(NK=16, Maxk=0.1)), ((32, 16, 64), 2, 1, 1, 0, 0, dict(NK=100, Maxk=0.05)),
+         ((32, 1024, 32), 1, 0, 0, 1, 1, dict(NK=9, Maxk=0.02)), ((32, 64, 32), 3, 2, 0, 0, 0, dict(NK=1, Maxk=0.2))]
 
 
 @pytest.mark.parametrize("precision", ["fp32", "det"])

@@ -1,4 +1,4 @@
-"""The FP32 survey estimator for power-of-two NX (64 to 1024), NY and NZ (weighted z pass, k_yfft, k_xrow_survey) against
+"""The FP32 survey estimator for power-of-two NX (32 to 1024), NY and NZ (weighted z pass, k_yfft, k_xrow_survey) against
 the oracle at the suite's tolerances: every row length, one, two and four slots, every (l, m), the observer off the grid
 and on a cell corner inside it, top edges below and beyond the Nyquist frequency, linear and logarithmic bins."""
 import pytest
@@ -14,7 +14,8 @@ CASES = [((64, 16, 32), 0, 3, 1, 1, 0, dict(NK=20, Maxk=1.2)), ((64, 64, 32), 2,
          ((256, 32, 32), 0, 1, 0, 1, 1, dict(NK=12, OutputLog=1, Mink=-1.6, Maxk=-0.2)),
          ((256, 16, 64), 2, 3, 1, 0, 0, dict(NK=10, Maxk=0.32)), ((512, 16, 32), 0, 3, 1, 1, 1, dict(NK=20, Maxk=0.6)),
          ((512, 32, 32), 3, 2, 1, 1, 0, dict(NK=16, Maxk=1.2)), ((1024, 32, 32), 0, 2, 1, 1, 0, dict(NK=9, Maxk=0.12)),
-         ((1024, 16, 32), 2, 1, 1, 0, 1, dict(NK=24, Maxk=0.8)), ((64, 256, 32), 1, 3, 0, 0, 1, dict(NK=1, Maxk=0.2))]
+         ((1024, 16, 32), 2, 1, 1, 0, 1, dict(NK=24, Maxk=0.8)), ((64, 256, 32), 1, 3, 0, 0, 1, dict(NK=1, Maxk=0.2)),
+         ((32, 32, 32), 0, 2, 1, 1, 1, dict(NK=16, Maxk=0.5)), ((32, 64, 64), 2, 3, 0, 1, 0, dict(NK=11, Maxk=0.4))]
 
 
 @pytest.mark.parametrize("shape,momentum,order,il,odd,corner,bins", CASES)

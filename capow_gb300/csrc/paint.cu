@@ -1774,6 +1774,7 @@ __global__ void __launch_bounds__(128) k_ovf_paint(Geom g, FieldSpec fs, TileGeo
                                                    GridPtrs grids, DevStats *st) {
   constexpr int NS = IL ? 2 : 1;
   const unsigned long long no = min((unsigned long long)*ovf_count, ovf_cap);
+  if (blockIdx.x * (unsigned long long)blockDim.x >= no) return;  // (most calls have none: no block sums then)
   double l_dc[4] = {0, 0, 0, 0};
   for (unsigned long long o = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; o < no;
        o += (unsigned long long)gridDim.x * blockDim.x) {
@@ -1834,6 +1835,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_edge_fixup(Geom g, FieldSpec fs, PIn<T> in, const unsigned *edge_list,
                                                     const unsigned *edge_count, GridPtrs grids, DevStats *st) {
   const unsigned ne = *edge_count;
+  if (blockIdx.x * (blockDim.x >> 5) >= ne) return;  // nothing for this CTA: no block sums
   const int nf = fs.nfields, nst = g.interlace ? 2 : 1;
   const int lane = threadIdx.x & 31;
   const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarp = (gridDim.x * blockDim.x) >> 5;

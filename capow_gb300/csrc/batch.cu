@@ -224,7 +224,24 @@ int setup_batch(BatchState *b, const capow_mock *mocks, int nmocks, const capow_
       capow_ctx *c = nullptr;
       capow_params cp = mocks[i].params;
       cp.InterpOrder = max_order[k];
-      const int r = capow_create(&cp, &so, &c);
+      int r = capow_create(&cp, &so, &c);
+      if (!r && c->blk) {  // every mock's bins have to fit the blocked x pass, else the context takes the other layouts
+        bool fit = true;
+        for (int j = 0; j < nmocks && fit; j++) {
+          if (b->status0[j] || shape_of(mocks[j].params) != k) continue;
+          BinParams q = c->bp;
+          XbinGeo xg;
+          q.nk = mocks[j].params.NK;
+          fit = xrow_plan(q, c->bt, c->nslot, xg);
+        }
+        if (!fit) {
+          capow_destroy(c);
+          c = nullptr;
+          ctx_no_blocked = true;
+          r = capow_create(&cp, &so, &c);
+          ctx_no_blocked = false;
+        }
+      }
       if (r) {
         if (c) capow_destroy(c);
         b->status0[i] = r;

@@ -9,9 +9,10 @@
 // modes within a few ulps of an edge. Mode counts do not depend on the fields and are
 // computed once per context by k_mode_counts.
 //
-// Accumulation: each thread walks the x axis of one (y, z) column; along a walk the bin
+// Accumulation (k_bin, k_bin64): each thread walks the x axis of one (y, z) column; along a walk the bin
 // changes rarely, so per-thread register sums of the current bin are flushed into shared
-// memory bins on a bin change, and each CTA adds its bins to the global FP64 sums.
+// memory bins on a bin change, and each CTA adds its bins to the global FP64 sums. The fused x axis +
+// binning kernels are k_xfft_bin here and, on the blocked path, k_xrow_bin (xrow.cuh).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
@@ -808,7 +809,7 @@ __global__ void __launch_bounds__(256) k_bin64(BinParams bp, BinTables t, const 
 }
 
 // ------------------------------------------------------------ fused x-axis FFT + binning (FP32)
-// Every x-plane of every grid has been transformed over (y, z) (by cuFFT in place, or by k_zr2c and
+// Every x-plane of every grid has been transformed over (y, z) (by cuFFT in place, or by k_zfft and
 // the y-axis C2C into the transposed layout); what is left of the 3-D transform (src/main.c:266-271)
 // is the length-NX DFT along x of every (ky, kz) column, and its only consumer is the binning
 // (src/main.c:302-468). One pass does both: a CTA transforms a block of columns along x in shared

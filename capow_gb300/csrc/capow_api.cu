@@ -13,6 +13,8 @@
 
 #include "ctx.cuh"
 
+thread_local bool ctx_no_blocked = false;
+
 extern "C" const char *capow_strerror(int s) {
   switch (s) {
     case CAPOW_OK: return "ok";
@@ -241,14 +243,14 @@ extern "C" int capow_create(const capow_params *p, const capow_options *opt, cap
     CK(c, cudaMemcpyAsync(c->nmodes2d.data(), c->nmodes2d_d, sizeof(unsigned long long) * n2d,
                           cudaMemcpyDeviceToHost, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
-  // FP32 with a power-of-two NX: the (y, z) axes first, then k_xfft_bin does the x axis together
+  // FP32 with a power-of-two NX: the (y, z) axes first, then k_xrow_bin or k_xfft_bin does the x axis together
   // with the binning (CAPOW_FFT_3D keeps the 3-D transform and k_bin). With a power-of-two NZ the z
-  // axis is k_zr2c, out of place and transposed to [NX][NZ/2+1][NY], and the y axis a contiguous
+  // axis is k_zfft, out of place and transposed to [NX][NZ/2+1][NY], and the y axis a contiguous
   // batched cuFFT C2C; otherwise one cuFFT 2-D R2C over every x-plane, in place.
   const bool want_fused = !f64 && o.fft_path != CAPOW_FFT_3D && c->bt.twx;
   const long long yrows = (long long)c->nslot * p->NX * bp.nzc;
   const bool tr = want_fused && c->bt.twz && zr2c_supported(bp) && yrows <= 0x7fffffffLL;
-  if (tr && o.fft_path == CAPOW_FFT_AUTO && xrow_plan(bp, c->bt, c->nslot, c->xg)) {
+  if (tr && !ctx_no_blocked && o.fft_path == CAPOW_FFT_AUTO && xrow_plan(bp, c->bt, c->nslot, c->xg)) {
     // power-of-two NY too: the blocked path. Its z and y passes run on up to 4 GB of planes at a time, so that a
     // large grid needs no third grid-sized buffer. (Each pair of launches costs about 20 us of ramps: at 512^3, runs
     // of planes that would stay in L2 between the passes took 1.76 ms at 64 MB and 2.7 ms at 32 MB, against 1.43 ms

@@ -39,7 +39,7 @@ struct capow_ctx {
   std::vector<unsigned long long> nmodes, nmodes2d;
   cufftHandle plan;
   bool plan_ok;
-  // transposed fused path (power-of-two NZ): k_zr2c writes [NX][NZ/2+1][NY] complex per slot into
+  // transposed fused path (power-of-two NZ): k_zfft writes [NX][NZ/2+1][NY] complex per slot into
   // tbuf, yplan is the batched C2C along y over it
   bool xtr;
   float2 *tbuf;
@@ -52,7 +52,7 @@ struct capow_ctx {
   int planes;
   float2 *ubuf;
   long long uslot;
-  // opt-in (CAPOW_FFT_ONE_LAUNCH): power-of-two NY as well: the z pass and the y axis in one launch (k_zy) instead of k_zr2c + yplan;
+  // opt-in (CAPOW_FFT_ONE_LAUNCH): power-of-two NY as well: the z pass and the y axis in one launch (k_zy) instead of k_zfft + yplan;
   // zy_ctr holds its work-queue and per-plane counters
   bool zy;
   unsigned *zy_ctr;
@@ -130,6 +130,9 @@ int create_paint_ctx(const capow_params *p, const capow_options *o, int survey, 
 // sync, read the paint counters into c->h_st, repaint c->last when the tile lists overflowed
 int settle_paint(capow_ctx *c);
 int enqueue_paint(capow_ctx *c, const capow_particles &d);
+// Set by a thread around capow_create: its context takes no blocked path. (A batch's mocks share contexts, and one whose
+// bins the blocked x pass cannot hold may fit the transposed one's.)
+extern thread_local bool ctx_no_blocked;
 int enqueue_power_kernels(capow_ctx *c);
 // Size the FP32 record and edge buffers (and, unless two_pass, the one-pass buckets at bucket_factor and
 // their overflow list) for catalogues of up to nmax particles, so that a later enqueue_paint allocates nothing.

@@ -5,8 +5,8 @@ Workload (the headline configuration): 256^3 = 16,777,216 Zel'dovich-displaced l
 density-density, density-momentum and momentum-momentum spectra from one paint, LOS = z (RSD shift),
 NK = 161 linear bins to k = 1.61 h/Mpc.
 
-One step = one full evaluation: paint (4 grids) -> z pass (k_zr2c) and cuFFT y pass -> fused x-axis
-FFT + bin kernel -> device-to-host copy of the bins. ``value`` times steps with the particles already
+One step = one full evaluation: paint (4 grids) -> z pass (k_zfft) and y pass (k_yfft) -> fused x-axis
+FFT + bin kernel (k_xrow_bin) -> device-to-host copy of the bins. ``value`` times steps with the particles already
 resident in HBM (CUDA events on the context stream, barrier + synchronize on both sides, max over
 ranks); ``e2e`` times the same evaluations through the public C-ABI calls with pinned HOST particle
 buffers, each step's host-to-device copy and read-back inside the timed region, as a stream of
@@ -48,8 +48,8 @@ SEED = 2
 PRECISION = ("fp32-mixed: FP32 grids, FFT, per-thread bin runs and per-CTA bin copies; FP64 global bin sums, "
              "scalars and near-edge indices; exact k-bins")
 # DRAM read + write bytes of one launch at this workload, from one ncu capture of it
-TRAFFIC_TILE_REC = 512893000 + 2119952000
-TRAFFIC_XFFT_BIN = 1768743000 + 3229000
+TRAFFIC_TILE_REC = 515440000 + 2120000000
+TRAFFIC_XROW_BIN = 1700000000 + 3520000
 
 
 def algorithmic_bytes(n_particles: int, ng: int, nc: int, grids: int, b_p: int, b_r: int, b_c: int) -> int:
@@ -855,17 +855,17 @@ def main():
         if r["r64"]:
             line["accuracy_vs_oracle"]["fp64"] = accuracy_vs_oracle(r["r64"], cpu["raw"])
     # the two largest kernels, each timed by the library's CUDA events on the context stream:
-    # k_tile_rec (the FP32 tile deposit; events around its one launch) and k_xfft_bin (x-axis FFT
+    # k_tile_rec (the FP32 tile deposit; events around its one launch) and k_xrow_bin (x-axis FFT
     # fused with the binning: the whole "bin" stage). "roofline" is the one that took longer.
     # k_tile_rec algorithmic bytes per launch: the four grids written once (NX NY NZ cells, 4 bytes)
     # plus one read of its particle records (16 bytes each; one record per particle and tile its
-    # stencils reach). k_xfft_bin: one read of the four (y,z)-transformed grids. Traffic: DRAM read
+    # stencils reach). k_xrow_bin: one read of the four (y,z)-transformed grids. Traffic: DRAM read
     # + write of one ncu capture of each at this workload.
     alg_t = 4 * 512 ** 3 * 4 + 16 * int(r["tile_records"])
     alg_x = 4 * 512 * 512 * 257 * 8
     rl = {}
     for name, alg, ms, traffic in (("k_tile_rec", alg_t, r["tile_ms"], TRAFFIC_TILE_REC),
-                                   ("k_xfft_bin", alg_x, bin_ms, TRAFFIC_XFFT_BIN)):
+                                   ("k_xrow_bin", alg_x, bin_ms, TRAFFIC_XROW_BIN)):
         ach = alg / (ms * 1e-3) / 1e9
         rl[name] = {"bound": "hbm", "kernel": name, "achieved": round(ach, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
                     "frac": round(ach / pk["hbm_gbs"], 4), "traffic": traffic, "algorithmic_bytes": alg,

@@ -1211,103 +1211,145 @@ __device__ __forceinline__ float store_pair(float *dst, float a0, float a1, bool
   return a0;
 }
 
-// A dense tile, one slot at a time: the records [r0, r1) of this CTA into cells of two int32 limbs (hi 2^17 + lo)
-// at a scale with (record count) (largest |w v^e|) 2^S < 2^47, which leaves a deposit its FP32 product for any
-// count; every 8192 records the low limbs' carries go to the high ones. Two native atomics a deposit: before
-// (int64 cells with 64-bit shared atomics, in chunks of a slot) 5.4M weighted particles took 32 ms into a 32^3
-// grid, 16.7M into 256^3 1.28 ms.
-constexpr int DENSE_K = 17;
-constexpr unsigned DENSE_ROUND = 8192;
+// A dense tile, one slot at a time: the records [r0, r1) of this CTA into cells of two int32 limbs, hi 2^K + lo, lo
+// unsigned: two native atomics a deposit. (int64 cells need 64-bit shared atomics, compare-and-swap loops: 5.4M weighted
+// particles, TSC, interlaced, into 32^3: 53 ms, by limbs 1.25 ms; 8M, CIC, interlaced, into 128^3: 0.57 and 0.43 ms. The
+// grids' errors against 64 bits are the same.) The scale is the finest that holds
+//  * every cell: the sum of |w v^e| 2^S below 2^49, so that a cell's high limb stays inside int32, and
+//  * every deposit: the largest |w v^e| 2^S below 2^41, so that its high limb stays inside rint_small's 2^22 (a share of a
+//    few hundred records lets one of them reach far into the sum's range).
+// Every 7936 records the low limbs' carries go to the high ones: 2^K plus 7936 deposits of up to 2^K fit 32 bits.
+// Where one record holds more than a quarter of the sum or 256 times the mean, the cells are int64 at 2^60 of the sum
+// instead, as slow as before. Elsewhere the quantum is below 2^-32 of the mean record (or 2^-48 of the sum), and the rounding
+// of the deposits stays below the rounding of the FP32 cell that they end in.
+constexpr int DENSE_K = 19;
+constexpr unsigned DENSE_ROUND = 7936;  // a multiple of the CTA's threads
 
+// Scale exponent of one field's cells: sum and max of |w v^e| over cnt records.
+__device__ __forceinline__ int dense_scale(float sum, float max, float cnt, bool &wide) {
+  const float sb = sum * 1.001f, mb = max * 1.001f;
+  wide = false;
+  if (!(sb > 0.0f) || !isfinite(sb)) return 0;
+  wide = max > 0.25f * sum || max * (cnt * 0x1p-8f) > sum;
+  const int es = ilogbf(sb), em = ilogbf(mb);  // sum < 2^(es + 1), max < 2^(em + 1)
+  const int S = wide ? 60 - es : min(48 - es, 40 - em);
+  return S > 100 ? 100 : (S < -100 ? -100 : S);
+}
+
+// Deposits of the records [r0, r1) into one slot's cells: WIDE: int64 cells at smi; otherwise the limbs lo, hi.
+template <int K, bool WIDE>
+__device__ __forceinline__ void dense_deposit(const Geom &g, const FieldSpec &fs, const TileGeo &tg, const float4 *recs,
+                                              const float *recw, unsigned long long r0, unsigned long long r1, int sten,
+                                              int fld, float sc, const TileAt &at, int *smi) {
+  int *lo = smi, *hi = smi + tg.slot;
+  const float two_k = (float)(1 << DENSE_K), two_mk = 1.0f / two_k;
+  for (unsigned long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+    const float4 rec = recs[r];
+    float va, vb;
+    record_values(fs, rec, recw ? recw[r] : 1.0f, va, vb);
+    const float v = (fld ? vb : va) * sc;
+    const float sx = sten ? __fadd_rn(rec.x, 0.5f) : rec.x, sy = sten ? __fadd_rn(rec.y, 0.5f) : rec.y,
+                sz = sten ? __fadd_rn(rec.z, 0.5f) : rec.z;
+    if (!accept32(g, sx, sy, sz)) continue;
+    AxisTapsF ax, ay, az;
+    axis32k<K>(sx, 0, g.nx, g.los, ax);
+    axis32k<K>(sy, 1, g.ny, g.los, ay);
+    axis32k<K>(sz, 1, g.nz, g.los, az);
+    float wx[3], wy[3], wz[3];
+    int ox[3], oy[3], oz[3];
+    stage_axis32(ax, at.x0, at.ex, tg.px, wx, ox);
+    stage_axis32(ay, at.y0, at.ey, tg.py, wy, oy);
+    stage_axis32(az, at.z0, at.ez, 1, wz, oz);
+#pragma unroll
+    for (int a = 0; a < K; a++)
+#pragma unroll
+      for (int b2 = 0; b2 < K; b2++) {
+        const float wxy = wx[a] * wy[b2];
+        if (wxy == 0.0f) continue;
+        const float pv = v * wxy;
+        const int oxy = ox[a] + oy[b2];
+#pragma unroll
+        for (int c = 0; c < K; c++) {
+          if (wz[c] == 0.0f) continue;
+          if (WIDE)
+            atomicAdd((unsigned long long *)smi + oxy + oz[c], (unsigned long long)__float2ll_rn(pv * wz[c]));
+          else
+            limb_add(lo + oxy + oz[c], hi + oxy + oz[c], pv * wz[c], two_mk, two_k);
+        }
+      }
+  }
+}
+
+// (r0, r1: this CTA's records of the tile's cnt; st4: sum |w v^ea|, sum |w v^eb|, and the two largest, over r0 to r1.) The
+// CTAs of a cluster take one scale, from the tile's sums, so that their cells add up as integers and a cell is rounded once.
 template <int K, int NF, bool IL, bool CL>
 __device__ void tile_paint_dense(const Geom &g, const FieldSpec &fs, const TileGeo &tg, const float4 *recs,
-                                 const float *recw, unsigned long long r0, unsigned long long r1, float xa, float xb,
-                                 const TileAt &at, int *smi, float *s_inv, GridPtrs grids, DevStats *st) {
+                                 const float *recw, unsigned long long r0, unsigned long long r1, unsigned cnt, float4 st4,
+                                 const TileAt &at, int *smi, float4 *s_stat, GridPtrs grids, DevStats *st) {
   constexpr int NS = IL ? 2 : 1;
   const int slotw = tg.slot;
   int *lo = smi, *hi = smi + slotw;
-  const float cnt = (float)(r1 - r0);
-  const float bound[2] = {cnt * xa * 1.001f, cnt * xb * 1.001f};
-  int Sx[2];
-#pragma unroll
-  for (int f = 0; f < 2; f++) {
-    const int S = bound[f] > 0.0f && isfinite(bound[f]) ? 46 - ilogbf(bound[f]) : 0;
-    Sx[f] = S > 100 ? 100 : (S < -100 ? -100 : S);
+  if (CL) {
+    if (threadIdx.x == 0) *s_stat = st4;
+    cluster_sync_all();
+    const unsigned q = (unsigned)__cvta_generic_to_shared(s_stat);
+    st4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int k = 0; k < at.S; k++) {
+      const unsigned p = map_cluster(q, k);
+      st4.x += ld_cluster_f32(p);
+      st4.y += ld_cluster_f32(p + 4);
+      st4.z = fmaxf(st4.z, ld_cluster_f32(p + 8));
+      st4.w = fmaxf(st4.w, ld_cluster_f32(p + 12));
+    }
   }
-  if (threadIdx.x == 0) {
-    s_inv[0] = ldexpf(1.0f, -Sx[0]);
-    s_inv[1] = ldexpf(1.0f, -Sx[1]);
-  }
-  const float two_k = (float)(1 << DENSE_K), two_mk = 1.0f / two_k;
+  bool wide[2];
+  const int Sx[2] = {dense_scale(st4.x, st4.z, (float)cnt, wide[0]), dense_scale(st4.y, st4.w, (float)cnt, wide[1])};
 #pragma unroll 1
   for (int slot = 0; slot < NS * NF; slot++) {
     const int sten = slot / NF, fld = slot % NF;
-    const float sc = ldexpf(1.0f, fld ? Sx[1] : Sx[0]);
+    const int S = fld ? Sx[1] : Sx[0];
+    const bool wd = fld ? wide[1] : wide[0];
+    const float sc = ldexpf(1.0f, S), inv = ldexpf(1.0f, -S);
     for (int c = threadIdx.x; c < 2 * slotw; c += blockDim.x) smi[c] = 0;
     __syncthreads();
-    for (unsigned long long rr = r0; rr < r1; rr += DENSE_ROUND) {
-      if (rr > r0) {  // carries of the records so far
-        __syncthreads();
-        for (int c = threadIdx.x; c < slotw; c += blockDim.x) {
-          const int v = lo[c];
-          hi[c] += v >> DENSE_K;
-          lo[c] = v & ((1 << DENSE_K) - 1);
-        }
-        __syncthreads();
-      }
-      const unsigned long long rt = min(r1, rr + DENSE_ROUND);
-      for (unsigned long long r = rr + threadIdx.x; r < rt; r += blockDim.x) {
-        const float4 rec = recs[r];
-        float va, vb;
-        record_values(fs, rec, recw ? recw[r] : 1.0f, va, vb);
-        const float v = (fld ? vb : va) * sc;
-        const float sx = sten ? __fadd_rn(rec.x, 0.5f) : rec.x, sy = sten ? __fadd_rn(rec.y, 0.5f) : rec.y,
-                    sz = sten ? __fadd_rn(rec.z, 0.5f) : rec.z;
-        if (!accept32(g, sx, sy, sz)) continue;
-        AxisTapsF ax, ay, az;
-        axis32k<K>(sx, 0, g.nx, g.los, ax);
-        axis32k<K>(sy, 1, g.ny, g.los, ay);
-        axis32k<K>(sz, 1, g.nz, g.los, az);
-        float wx[3], wy[3], wz[3];
-        int ox[3], oy[3], oz[3];
-        stage_axis32(ax, at.x0, at.ex, tg.px, wx, ox);
-        stage_axis32(ay, at.y0, at.ey, tg.py, wy, oy);
-        stage_axis32(az, at.z0, at.ez, 1, wz, oz);
-#pragma unroll
-        for (int a = 0; a < K; a++)
-#pragma unroll
-          for (int b2 = 0; b2 < K; b2++) {
-            const float wxy = wx[a] * wy[b2];
-            if (wxy == 0.0f) continue;
-            const float pv = v * wxy;
-            const int oxy = ox[a] + oy[b2];
-#pragma unroll
-            for (int c = 0; c < K; c++)
-              if (wz[c] != 0.0f) limb_add(lo + oxy + oz[c], hi + oxy + oz[c], pv * wz[c], two_mk, two_k);
+    if (wd) {
+      dense_deposit<K, true>(g, fs, tg, recs, recw, r0, r1, sten, fld, sc, at, smi);
+    } else {
+      for (unsigned long long rr = r0; rr < r1; rr += DENSE_ROUND) {
+        if (rr > r0) {  // carries of the records so far
+          __syncthreads();
+          for (int c = threadIdx.x; c < slotw; c += blockDim.x) {
+            const unsigned v = (unsigned)lo[c];
+            hi[c] += (int)(v >> DENSE_K);
+            lo[c] = (int)(v & ((1u << DENSE_K) - 1));
           }
+          __syncthreads();
+        }
+        dense_deposit<K, false>(g, fs, tg, recs, recw, rr, min(r1, rr + DENSE_ROUND), sten, fld, sc, at, smi);
       }
     }
     if (CL) cluster_sync_all();
     else __syncthreads();
     float *gp = (float *)grids.g[slot];
     float dsum = 0.0f;
-    const unsigned la = (unsigned)__cvta_generic_to_shared(lo), ha = (unsigned)__cvta_generic_to_shared(hi),
-                   ia = (unsigned)__cvta_generic_to_shared(s_inv + fld);
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smi);
+    // a cell's two words (low, high) lie dh apart, the next cell's dc further on
+    const int sh = wd ? 32 : DENSE_K, dh = wd ? 1 : slotw, dc = wd ? 2 : 1;
+    auto value = [sh](int l, int h) { return ((long long)h << sh) + (long long)(unsigned)l; };
     tile_walk<CL>(g, tg, at, [&](int cp, long long go, bool two) {
-      float a0 = 0.0f, a1 = 0.0f;
+      long long v0 = 0, v1 = 0;
       if (CL) {
         for (int k = 0; k < at.S; k++) {
-          const unsigned l = map_cluster(la, k) + 4 * cp, h = map_cluster(ha, k) + 4 * cp;
-          const float inv = ld_cluster_f32(map_cluster(ia, k));
-          a0 += (float)(((long long)ld_cluster_s32(h) << DENSE_K) + ld_cluster_s32(l)) * inv;
-          a1 += (float)(((long long)ld_cluster_s32(h + 4) << DENSE_K) + ld_cluster_s32(l + 4)) * inv;
+          const unsigned q = map_cluster(sa, k) + 4 * dc * cp;
+          v0 += value(ld_cluster_s32(q), ld_cluster_s32(q + 4 * dh));
+          v1 += value(ld_cluster_s32(q + 4 * dc), ld_cluster_s32(q + 4 * (dc + dh)));
         }
       } else {
-        const float inv = ldexpf(1.0f, -(fld ? Sx[1] : Sx[0]));
-        a0 = (float)(((long long)hi[cp] << DENSE_K) + lo[cp]) * inv;
-        a1 = (float)(((long long)hi[cp + 1] << DENSE_K) + lo[cp + 1]) * inv;
+        const int *q = smi + dc * cp;
+        v0 = value(q[0], q[dh]);
+        v1 = value(q[dc], q[dc + dh]);
       }
-      dsum += store_pair(gp + go, a0, a1, two);
+      dsum += store_pair(gp + go, (float)v0 * inv, (float)v1 * inv, two);
     });
     const float vals[1] = {dsum};
     double *const dst1[1] = {&st->dc[slot]};
@@ -1380,6 +1422,7 @@ __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileG
   // pre-pass over the records: sum and largest |w v^e| per field (the records stay in L1 for the deposits)
   __shared__ float red_abs[4][8];
   __shared__ float s_inv[2];  // 1 / scale of the CTA's cells per field
+  __shared__ float4 s_stat;   // (dense tiles) the sums and largest values below
   {
     float la = 0.0f, lb = 0.0f, ma = 0.0f, mb = 0.0f;
     auto add = [&](const float4 &rec, float w) {
@@ -1418,7 +1461,8 @@ __global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileG
     xb = fmaxf(xb, red_abs[3][k]);
   }
   if (cnt > dense) {  // uniform over the tile's CTAs
-    tile_paint_dense<K, NF, IL, CL>(g, fs, tg, recs, recw, rb, re, xa, xb, at, smi, s_inv, grids, st);
+    tile_paint_dense<K, NF, IL, CL>(g, fs, tg, recs, recw, rb, re, cnt, make_float4(ta, tb, xa, xb), at, smi, &s_stat, grids,
+                                    st);
     return;
   }
   // The scale is set by the sum (tile_scale_exp). When keeping every deposit below 2^22 costs

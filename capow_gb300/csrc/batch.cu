@@ -21,6 +21,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "ctx.cuh"
@@ -80,13 +81,16 @@ int time_paint(capow_ctx *c, const capow_particles &d, float *ms) {
   return rc;
 }
 
-// tile shapes and bucket factors chosen by the autotuner, per grid shape, for the life of the process
+// tile shapes and bucket factors chosen by the autotuner, per grid shape and number of painted slots, for the life of the
+// process. (The slots follow from the requested spectra too, which the shape does not hold; a shape tuned for four slots has
+// up to twice the tiles that a context of two has tables for.)
 struct Tuned {
   TileGeo tg;
   float bucket_factor;
 };
+typedef std::pair<ShapeKey, int> TunedKey;
 std::mutex g_tuned_mu;
-std::map<ShapeKey, Tuned> g_tuned;
+std::map<TunedKey, Tuned> g_tuned;
 
 // Bucket capacity factors the autotuner times (records per tile = factor * mean share + 64): smaller
 // buckets write fewer record slots, larger ones send fewer records to the slower overflow path.
@@ -340,8 +344,8 @@ int setup_batch(BatchState *b, const capow_mock *mocks, int nmocks, const capow_
     if (!(flags & CAPOW_BATCH_AUTOTUNE) || c->prec != CAPOW_FP32_MIXED) continue;
     {
       std::lock_guard<std::mutex> lock(g_tuned_mu);
-      auto it = g_tuned.find(kv.first);
-      if (it != g_tuned.end()) {
+      auto it = g_tuned.find(TunedKey(kv.first, c->nslot));
+      if (it != g_tuned.end() && it->second.tg.ntiles <= c->tg.ntiles) {
         for (capow_ctx *r : kv.second) {
           r->tg = it->second.tg;
           r->bucket_factor = it->second.bucket_factor;
@@ -387,7 +391,7 @@ int setup_batch(BatchState *b, const capow_mock *mocks, int nmocks, const capow_
       r->bucket_factor = best_f;
     }
     std::lock_guard<std::mutex> lock(g_tuned_mu);
-    g_tuned[kv.first] = Tuned{best, best_f};
+    g_tuned[TunedKey(kv.first, c->nslot)] = Tuned{best, best_f};
   }
   for (capow_ctx *c : b->all) {  // the buffers for the chosen tiles and buckets: enqueues allocate nothing
     int rc = prepare_paint_buffers(c, nmax[c], wts[c]);

@@ -1893,7 +1893,7 @@ static void launch_zy_t(cudaStream_t s, const ZyGeo &yg, const BinTables &t, con
   const unsigned M = 1u << yg.zg.log2m, ny = 1u << yg.log2ny;
   const unsigned zdata = zy_zdata_bytes(yg.zg.log2m, ZB), ydata = align16(8u * ZY_KB * (ny + ny / 8));
   const size_t smem = (zdata > ydata ? zdata : ydata) + zr2c_tables_bytes(yg.zg.log2m) + zy_ytables_bytes(yg.log2ny);
-  const int resident = resident_ctas((const void *)k_zy<ZB>, ZR_THREADS, smem);
+  const int resident = resident_ctas((const void *)k_zy<ZB>, ZR_THREADS, smem, 64);
   long long grid = resident;
   if (grid > yg.nitems) grid = yg.nitems;
   k_zy<ZB><<<(unsigned)grid, ZR_THREADS, smem, s>>>(yg, t, in, out, ctr, st);
@@ -2020,10 +2020,10 @@ void launch_mode_counts(cudaStream_t s, const BinParams &bp, const BinTables &t,
   const size_t smem = 8u * (size_t)bp.nk + 16u * (size_t)(bp.nk + 3);
   if (bp.out2d || smem > 200 * 1024) {
     const size_t each = sizeof(unsigned long long) * (bp.nk + (bp.out2d ? bp.nk * bp.nmu : 0));
-    cudaFuncSetAttribute(k_mode_counts_each, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each);
+    allow_smem(k_mode_counts_each);
     k_mode_counts_each<<<152 * 4, 256, each, s>>>(bp, t, nmodes, nmodes2d);
   } else {
-    cudaFuncSetAttribute(k_mode_counts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_mode_counts);
     const long long ncol = (long long)(bp.ny / 2 + 1) * (bp.kzmax + 1);  // a column per warp at least
     k_mode_counts<<<(unsigned)std::min<long long>(152 * 4, (ncol + 7) / 8), 256, smem, s>>>(bp, t, nmodes);
   }
@@ -2054,7 +2054,7 @@ static void launch_bin_t(cudaStream_t s, const BinParams &bp, const BinTables &t
   const int n2d = OUT2D ? bp.nk * bp.nmu : 0;
   const int sm2d = (size_t)(NP * n2d) * sizeof(R) <= 64 * 1024 ? 1 : 0;
   const size_t smem = bin_smem_layout(sizeof(R), NP, bp.nk, sm2d ? n2d : 0, ichunk).total;
-  cudaFuncSetAttribute(k_bin<R, NF, ODD, OUT2D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_bin<R, NF, ODD, OUT2D>);
   // slot order: stencil * nfields + field
   const C *gA = (const C *)slots[0];
   const C *gB = NF == 2 ? (const C *)slots[1] : nullptr;
@@ -2074,7 +2074,7 @@ static void launch_bin64(cudaStream_t s, const BinParams &bp, const BinTables &t
   const int ichunk = (half + nchunk - 1) / nchunk;
   nchunk = (half + ichunk - 1) / ichunk;
   const size_t smem = bin_smem_layout(8, NF == 1 ? 1 : 4, bp.nk, 0, ichunk).total;
-  cudaFuncSetAttribute(k_bin64<NF, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_bin64<NF, ODD>);
   const bool il = bp.interlace != 0;
   k_bin64<NF, ODD><<<dim3(nbx, nchunk), 256, smem, s>>>(
       bp, t, (const double2 *)slots[0], NF == 2 ? (const double2 *)slots[1] : nullptr,

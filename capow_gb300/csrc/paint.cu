@@ -216,7 +216,7 @@ static void launch_paint64_t(cudaStream_t s, const Geom &g, const FieldSpec &fs,
                              const GridPtrs &grids, DevStats *st) {
   auto *fn = g.order == 1 ? k_paint64<T, 1> : (g.order == 2 ? k_paint64<T, 2> : k_paint64<T, 3>);
   // one resident wave: each CTA ends with a reduction of twelve FP64 sums
-  const int nb = std::min(grid_blocks(n, 256), resident_ctas((const void *)fn, 256, 0));
+  const int nb = std::min(grid_blocks(n, 256), resident_ctas((const void *)fn, 256, 0, 4096));
   fn<<<nb, 256, 0, s>>>(g, fs, in, n, grids, st);
 }
 
@@ -955,7 +955,7 @@ static void launch_bucket(cudaStream_t s, const Geom &g, const FieldSpec &fs, co
                       b.ovf_tile, b.ovf_count,             b.ovf_cap};
   if (tg.ntiles <= BK_DIRECT_TILES) {
     const size_t smem = bucket_smem(tg.ntiles);
-    cudaFuncSetAttribute(k_bucket_cta<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_bucket_cta<T>, 8192);
     // one resident wave (two CTAs per SM); a small catalogue takes fewer particles per chunk, to fill it
     const long long wave = 152LL * 2 * BK_THREADS;
     const int ppt = (int)std::min<long long>(BK_PPT, std::max<long long>(1, n / wave));
@@ -2027,7 +2027,7 @@ static void launch_rec(cudaStream_t s, const Geom &g, const FieldSpec &fs, const
   const unsigned dense = (unsigned)((double)TILE_DENSE_RECORDS * std::min(1.0, (double)tg.tx * tg.ty * tg.tz /
                                                                                ((double)def.tx * def.ty * def.tz)));
   if (split > 1) {
-    cudaFuncSetAttribute(k_tile_rec<K, NF, IL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_tile_rec<K, NF, IL, true>, 4096);
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = (unsigned)split;
@@ -2043,7 +2043,7 @@ static void launch_rec(cudaStream_t s, const Geom &g, const FieldSpec &fs, const
                        (const unsigned *)b.counts, b.bucket_cap, (const float4 *)b.recs, recw, b.capacity, split, dense,
                        grids, st);
   } else {
-    cudaFuncSetAttribute(k_tile_rec<K, NF, IL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_tile_rec<K, NF, IL, false>, 4096);
     k_tile_rec<K, NF, IL, false><<<tg.ntiles, 256, smem, s>>>(g, fs, tg, b.offsets, b.counts, b.bucket_cap, b.recs,
                                                                    recw, b.capacity, 1, dense, grids, st);
   }
@@ -2068,7 +2068,7 @@ template <typename T, int K, int NF, bool IL>
 static void launch_det(cudaStream_t s, const Geom &g, const FieldSpec &fs, const TileGeo &tg, const PIn<T> &in,
                        long long n, const PaintBufs &b, const GridPtrs &grids, DevStats *st) {
   const size_t smem = tile_smem_bytes(tg, NF, 1);
-  cudaFuncSetAttribute(k_tile_rec_det<T, K, NF, IL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_tile_rec_det<T, K, NF, IL>, 4096);
   k_tile_rec_det<T, K, NF, IL><<<tg.ntiles, 256, smem, s>>>(g, fs, tg, in, n, b.offsets, b.recs,
                                                             in.w ? b.recw : nullptr, b.capacity, grids, b.fixed_scale,
                                                             st);

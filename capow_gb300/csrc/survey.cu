@@ -44,6 +44,7 @@
 
 #include "ctx.cuh"
 #include "harm.cuh"
+#include "launch.cuh"
 
 // ------------------------------------------------------------------------------------ device state
 struct SvStats {
@@ -1357,7 +1358,7 @@ static int sv_paint_tiles(capow_survey_ctx *c, const capow_survey_catalogue *dat
       const SvBounds bd = sv_bounds(c->g);
       if constexpr (sizeof(T) == 4) {
         if (part) {
-          cudaFuncSetAttribute(k_sv_partition32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SV_PART_SMEM);
+          allow_smem(k_sv_partition32, 4096);
           const long long nb = (m + SV_PART_CH - 1) / SV_PART_CH;
           k_sv_partition32<<<(unsigned)std::min<long long>(nb, 152 * 2), SV_PART_T, SV_PART_SMEM, c->stream>>>(
               bd, pt, sin, wk, m, cat, c->part, cx, cy, cz, cw, c->st);

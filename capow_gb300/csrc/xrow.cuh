@@ -370,7 +370,7 @@ static void launch_xrow_n(cudaStream_t s, const BinParams &bp, const BinTables &
                           void *const slots[4], const double *dcv, double *bins) {
   constexpr int NS = NF * (IL ? 2 : 1);
   const size_t smem = xrow_smem_layout(LN, NS, xrow_products(bp), xrow_multipoles(bp), bp.nk, xg.nbc).total;
-  int grid = resident_ctas((const void *)k_xrow_bin<NF, IL, ODD, PM, LN>, xr_threads(LN), smem);
+  int grid = resident_ctas((const void *)k_xrow_bin<NF, IL, ODD, PM, LN>, xr_threads(LN), smem, 64);
   if (grid > xg.nblocks) grid = xg.nblocks;
   k_xrow_bin<NF, IL, ODD, PM, LN><<<grid, xr_threads(LN), smem, s>>>(bp, t, xg, (const float2 *)slots[0],
                                                                  (const float2 *)slots[1], (const float2 *)slots[2],

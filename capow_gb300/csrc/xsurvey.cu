@@ -198,7 +198,7 @@ static void launch_xs_n(cudaStream_t s, const BinParams &bp, const BinTables &t,
                         long long uslot, const SvSet &set, double *bins) {
   constexpr int NS = NF * (IL ? 2 : 1);
   const size_t smem = xrow_smem_layout(LN, NS, 1, xs_sums(LZ), bp.nk, xg.nbc).total;
-  int grid = resident_ctas((const void *)k_xrow_survey<NF, IL, LZ, LN>, xr_threads(LN), smem);
+  int grid = resident_ctas((const void *)k_xrow_survey<NF, IL, LZ, LN>, xr_threads(LN), smem, 64);
   if (grid > xg.nblocks) grid = xg.nblocks;
   k_xrow_survey<NF, IL, LZ, LN><<<grid, xr_threads(LN), smem, s>>>(bp, t, xg, u, u + uslot, u + 2 * uslot, u + 3 * uslot, set,
                                                                 bins);

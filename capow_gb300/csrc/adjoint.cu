@@ -596,10 +596,21 @@ static int make_3d_plans(capow_ctx *c) {
   int inembed[3] = {p->NX, p->NY, 2 * nzc}, onembed[3] = {p->NX, p->NY, nzc};
   const long long idist = (long long)c->grid_elems, odist = (long long)c->grid_elems / 2;
   if (idist > 0x7fffffffLL) FAIL(c, CAPOW_ENOTSUP, "capow_backward: grid too large for one batched plan");
-  CKFFT(c, cufftPlanMany(&c->adj_fwd, 3, n, inembed, 1, (int)idist, onembed, 1, (int)odist, f64 ? CUFFT_D2Z : CUFFT_R2C,
-                         c->nslot));
-  CKFFT(c, cufftPlanMany(&c->adj_inv, 3, n, onembed, 1, (int)odist, inembed, 1, (int)idist, f64 ? CUFFT_Z2D : CUFFT_C2R,
-                         c->nslot));
+  auto forward = [&] {
+    return cufftPlanMany(&c->adj_fwd, 3, n, inembed, 1, (int)idist, onembed, 1, (int)odist, f64 ? CUFFT_D2Z : CUFFT_R2C,
+                         c->nslot);
+  };
+  auto inverse = [&] {
+    return cufftPlanMany(&c->adj_inv, 3, n, onembed, 1, (int)odist, inembed, 1, (int)idist, f64 ? CUFFT_Z2D : CUFFT_C2R,
+                         c->nslot);
+  };
+  // (no room for a plan's workspace: once more without the blocked layout's buffers)
+  cufftResult r = forward();
+  if (r != CUFFT_SUCCESS && leave_blocked(c)) r = forward();
+  CKFFT(c, r);
+  r = inverse();
+  if (r != CUFFT_SUCCESS && leave_blocked(c)) r = inverse();
+  CKFFT(c, r);
   CKFFT(c, cufftSetStream(c->adj_fwd, c->stream));
   CKFFT(c, cufftSetStream(c->adj_inv, c->stream));
   c->adj_plans = true;
@@ -710,7 +721,7 @@ extern "C" int capow_backward(capow_ctx *c, const double *const *dL_dP, const ca
   // device: the coefficients in FP64, Re Gamma(0) of the density's two slots, the coefficients in FP32
   const size_t ncoef = (size_t)NPROD * 5 * nk;
   if (!c->adj_coef)
-    CK(c, cudaMalloc(&c->adj_coef, sizeof(double) * (ncoef + 2) + sizeof(float) * ncoef));
+    CK(c, ctx_malloc(c, (void **)&c->adj_coef, sizeof(double) * (ncoef + 2) + sizeof(float) * ncoef));
   double *coef_d = c->adj_coef, *gamma0 = c->adj_coef + ncoef;
   float *coef_f = (float *)(c->adj_coef + ncoef + 2);
   CK(c, cudaMemcpyAsync(coef_d, coef.data(), sizeof(double) * ncoef, cudaMemcpyHostToDevice, c->stream));
@@ -753,7 +764,7 @@ extern "C" int capow_backward(capow_ctx *c, const double *const *dL_dP, const ca
         if (c->adj_stage[k]) cudaFree(c->adj_stage[k]);
         c->adj_stage[k] = nullptr;
         c->adj_stage_bytes[k] = 0;
-        CK(c, cudaMalloc(&c->adj_stage[k], ob * (size_t)(n ? n : 1)));
+        CK(c, ctx_malloc(c, (void **)&c->adj_stage[k], ob * (size_t)(n ? n : 1)));
         c->adj_stage_bytes[k] = ob * (size_t)(n ? n : 1);
       }
       dev[k] = c->adj_stage[k];

@@ -465,6 +465,19 @@ extern "C" int capow_batch(capow_mock *mocks, int nmocks, const capow_options *o
     if (!b) return CAPOW_ENOMEM;
     b->sig = sig;
     rc = setup_batch(b, mocks, nmocks, o, flags);
+    bool failed = rc != CAPOW_OK, blocked = false;
+    for (int st : b->status0) failed = failed || st == CAPOW_ENOMEM || st == CAPOW_ECUDA || st == CAPOW_ECUFFT;
+    for (capow_ctx *c : b->all) blocked = blocked || c->blk;
+    if (failed && blocked) {  // perhaps for want of memory: once more without the blocked layout's buffers
+      free_batch_state(b);
+      (void)cudaGetLastError();
+      b = new (std::nothrow) BatchState();
+      if (!b) return CAPOW_ENOMEM;
+      b->sig = sig;
+      ctx_no_blocked = true;
+      rc = setup_batch(b, mocks, nmocks, o, flags);
+      ctx_no_blocked = false;
+    }
     if (rc) {
       free_batch_state(b);
       return rc;

@@ -163,6 +163,128 @@ static void *dalloc(capow_ctx *c, size_t bytes) {
   return p;
 }
 
+// The transform layout of a context whose tables and grids stand, and its buffers and plan. blocked: the blocked layout may
+// be taken.
+static int choose_layout(capow_ctx *c, bool blocked) {
+  // FP32 with a power-of-two NX: the (y, z) axes first, then k_xrow_bin or k_xfft_bin does the x axis together
+  // with the binning (CAPOW_FFT_3D keeps the 3-D transform and k_bin). With a power-of-two NZ the z
+  // axis is k_zfft, out of place and transposed to [NX][NZ/2+1][NY], and the y axis a contiguous
+  // batched cuFFT C2C; otherwise one cuFFT 2-D R2C over every x-plane, in place.
+  const capow_params *p = &c->p;
+  const capow_options &o = c->o;
+  const BinParams &bp = c->bp;
+  const bool f64 = c->prec == CAPOW_FP64;
+  const bool want_fused = !f64 && o.fft_path != CAPOW_FFT_3D && c->bt.twx;
+  const long long yrows = (long long)c->nslot * p->NX * bp.nzc;
+  const bool tr = want_fused && c->bt.twz && zr2c_supported(bp) && yrows <= 0x7fffffffLL;
+  if (tr && blocked && o.fft_path == CAPOW_FFT_AUTO && xrow_plan(bp, c->bt, c->nslot, c->xg)) {
+    // power-of-two NY too: the blocked path. Its z and y passes run on up to 4 GB of planes at a time, so that a
+    // large grid needs no third grid-sized buffer. (Each pair of launches costs about 20 us of ramps: at 512^3, runs
+    // of planes that would stay in L2 between the passes took 1.76 ms at 64 MB and 2.7 ms at 32 MB, against 1.43 ms
+    // for one of each.) These planes are memory that the transposed layout does not take; the context gives both buffers
+    // back when a later allocation finds no room (leave_blocked).
+    const long long plane = (long long)bp.nzc * p->NY;
+    // (a multiple of 64: the y pass writes runs of 16 planes)
+    c->planes = (int)std::min<long long>(p->NX, std::max<long long>(1, (4LL << 30) / (8 * plane * c->nslot) / 64) * 64);
+    c->tslot = plane * c->planes;
+    c->uslot = plane * p->NX;
+    void *tb = nullptr, *ub = nullptr;
+    if (cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess &&
+        cudaMalloc(&ub, sizeof(float2) * (size_t)c->uslot * c->nslot) == cudaSuccess) {
+      c->tbuf = (float2 *)tb;
+      c->ubuf = (float2 *)ub;
+      c->fused = c->xtr = c->blk = true;
+      c->plan_ok = true;  // the context is complete (no cuFFT plan on this path)
+      return CAPOW_OK;
+    }
+    if (tb) cudaFree(tb);
+    (void)cudaGetLastError();  // no room: the layouts below
+  }
+  c->fused = want_fused && xbin_plan(bp, c->nslot, c->xg, tr);
+  if (c->fused && tr) {
+    // the transposed layout needs a second grid-sized buffer and a cuFFT workspace; when the device
+    // has no room for them the context keeps the in-place 2-D cuFFT layout instead
+    c->tslot = (long long)p->NX * bp.nzc * p->NY;
+    void *tb = nullptr;
+    int ny = p->NY;
+    if (o.fft_path == CAPOW_FFT_ONE_LAUNCH && zy_supported(bp, c->bt)) {  // z and y axes in one launch
+      const char *stall = getenv("CAPOW_TEST_STALL_ZY");
+      c->zy_stall = stall && stall[0] == '1';
+      c->zy_ctr = (unsigned *)dalloc(c, sizeof(unsigned) * zy_counter_words(bp, c->nslot));
+      if (c->zy_ctr && cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess) {
+        c->allocs.push_back(tb);
+        c->tbuf = (float2 *)tb;
+        c->xtr = true;
+        c->zy = true;
+        c->plan_ok = true;
+        return CAPOW_OK;
+      }
+      tb = nullptr;
+    }
+    if (cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess) {
+      if (cufftPlanMany(&c->yplan, 1, &ny, nullptr, 1, ny, nullptr, 1, ny, CUFFT_C2C, (int)yrows) == CUFFT_SUCCESS) {
+        c->allocs.push_back(tb);
+        c->tbuf = (float2 *)tb;
+        c->xtr = true;
+        c->yplan_ok = true;
+        CKFFT(c, cufftSetStream(c->yplan, c->stream));
+        c->plan_ok = true;  // the context is complete (c->plan is not used on this path)
+        return CAPOW_OK;
+      }
+      cudaFree(tb);
+    }
+    (void)cudaGetLastError();  // clear the failed allocation
+    c->fused = xbin_plan(bp, c->nslot, c->xg, false);
+  }
+  if (c->fused) {
+    int n2[2] = {p->NY, p->NZ};
+    int in2[2] = {p->NY, 2 * bp.nzc}, on2[2] = {p->NY, bp.nzc};
+    CKFFT(c, cufftPlanMany(&c->plan, 2, n2, in2, 1, p->NY * 2 * bp.nzc, on2, 1, p->NY * bp.nzc, CUFFT_R2C,
+                           p->NX * c->nslot));
+    c->plan_ok = true;
+    CKFFT(c, cufftSetStream(c->plan, c->stream));
+    return CAPOW_OK;
+  }
+  // one batched in-place r2c plan over all painted grids (replaces the fftw_execute calls,
+  // src/main.c:266-271): forward, unnormalised, padded last dimension
+  int n[3] = {p->NX, p->NY, p->NZ};
+  int inembed[3] = {p->NX, p->NY, 2 * bp.nzc}, onembed[3] = {p->NX, p->NY, bp.nzc};
+  long long idist = (long long)c->grid_elems, odist = (long long)c->grid_elems / 2;
+  if (idist > 0x7fffffffLL) {
+    // cufftPlanMany takes int distances; large grids use one plan per grid instead
+    CKFFT(c, cufftPlan3d(&c->plan, p->NX, p->NY, p->NZ, f64 ? CUFFT_D2Z : CUFFT_R2C));
+  } else {
+    CKFFT(c, cufftPlanMany(&c->plan, 3, n, inembed, 1, (int)idist, onembed, 1, (int)odist,
+                           f64 ? CUFFT_D2Z : CUFFT_R2C, c->nslot));
+  }
+  c->plan_ok = true;
+  CKFFT(c, cufftSetStream(c->plan, c->stream));
+  return CAPOW_OK;
+}
+
+// The blocked layout holds up to 4 GB more than the transposed one. When an allocation after capow_create finds no room, the
+// context gives its buffers back and takes the layout that it would have had without it. False: it has none to give
+// back (a batch's contexts keep theirs: the mocks' bins are planned for the layout, and the batch is set up again instead).
+bool leave_blocked(capow_ctx *c) {
+  if (!c->blk || c->quiet) return false;
+  (void)cudaGetLastError();
+  cudaStreamSynchronize(c->stream);  // a queued power stage reads them
+  cudaFree(c->tbuf);
+  cudaFree(c->ubuf);
+  c->tbuf = c->ubuf = nullptr;
+  c->fused = c->xtr = c->blk = c->plan_ok = false;
+  const int rc = choose_layout(c, false);
+  (void)cudaGetLastError();
+  return rc == CAPOW_OK;
+}
+
+// cudaMalloc of a buffer that a context needs after its creation.
+cudaError_t ctx_malloc(capow_ctx *c, void **q, size_t bytes) {
+  cudaError_t e = cudaMalloc(q, bytes);
+  if (e == cudaErrorMemoryAllocation && leave_blocked(c)) e = cudaMalloc(q, bytes);
+  return e;
+}
+
 extern "C" int capow_create(const capow_params *p, const capow_options *opt, capow_ctx **out) {
   if (!p || !out) return CAPOW_EINVAL;
   *out = nullptr;
@@ -243,97 +365,7 @@ extern "C" int capow_create(const capow_params *p, const capow_options *opt, cap
     CK(c, cudaMemcpyAsync(c->nmodes2d.data(), c->nmodes2d_d, sizeof(unsigned long long) * n2d,
                           cudaMemcpyDeviceToHost, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
-  // FP32 with a power-of-two NX: the (y, z) axes first, then k_xrow_bin or k_xfft_bin does the x axis together
-  // with the binning (CAPOW_FFT_3D keeps the 3-D transform and k_bin). With a power-of-two NZ the z
-  // axis is k_zfft, out of place and transposed to [NX][NZ/2+1][NY], and the y axis a contiguous
-  // batched cuFFT C2C; otherwise one cuFFT 2-D R2C over every x-plane, in place.
-  const bool want_fused = !f64 && o.fft_path != CAPOW_FFT_3D && c->bt.twx;
-  const long long yrows = (long long)c->nslot * p->NX * bp.nzc;
-  const bool tr = want_fused && c->bt.twz && zr2c_supported(bp) && yrows <= 0x7fffffffLL;
-  if (tr && !ctx_no_blocked && o.fft_path == CAPOW_FFT_AUTO && xrow_plan(bp, c->bt, c->nslot, c->xg)) {
-    // power-of-two NY too: the blocked path. Its z and y passes run on up to 4 GB of planes at a time, so that a
-    // large grid needs no third grid-sized buffer. (Each pair of launches costs about 20 us of ramps: at 512^3, runs
-    // of planes that would stay in L2 between the passes took 1.76 ms at 64 MB and 2.7 ms at 32 MB, against 1.43 ms
-    // for one of each.)
-    const long long plane = (long long)bp.nzc * p->NY;
-    // (a multiple of 64: the y pass writes runs of 16 planes)
-    c->planes = (int)std::min<long long>(p->NX, std::max<long long>(1, (4LL << 30) / (8 * plane * c->nslot) / 64) * 64);
-    c->tslot = plane * c->planes;
-    c->uslot = plane * p->NX;
-    void *tb = nullptr, *ub = nullptr;
-    if (cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess &&
-        cudaMalloc(&ub, sizeof(float2) * (size_t)c->uslot * c->nslot) == cudaSuccess) {
-      c->allocs.push_back(tb);
-      c->allocs.push_back(ub);
-      c->tbuf = (float2 *)tb;
-      c->ubuf = (float2 *)ub;
-      c->fused = c->xtr = c->blk = true;
-      c->plan_ok = true;  // the context is complete (no cuFFT plan on this path)
-      return CAPOW_OK;
-    }
-    if (tb) cudaFree(tb);
-    (void)cudaGetLastError();  // no room: the layouts below
-  }
-  c->fused = want_fused && xbin_plan(bp, c->nslot, c->xg, tr);
-  if (c->fused && tr) {
-    // the transposed layout needs a second grid-sized buffer and a cuFFT workspace; when the device
-    // has no room for them the context keeps the in-place 2-D cuFFT layout instead
-    c->tslot = (long long)p->NX * bp.nzc * p->NY;
-    void *tb = nullptr;
-    int ny = p->NY;
-    if (o.fft_path == CAPOW_FFT_ONE_LAUNCH && zy_supported(bp, c->bt)) {  // z and y axes in one launch
-      const char *stall = getenv("CAPOW_TEST_STALL_ZY");
-      c->zy_stall = stall && stall[0] == '1';
-      c->zy_ctr = (unsigned *)dalloc(c, sizeof(unsigned) * zy_counter_words(bp, c->nslot));
-      if (c->zy_ctr && cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess) {
-        c->allocs.push_back(tb);
-        c->tbuf = (float2 *)tb;
-        c->xtr = true;
-        c->zy = true;
-        c->plan_ok = true;
-        return CAPOW_OK;
-      }
-      tb = nullptr;
-    }
-    if (cudaMalloc(&tb, sizeof(float2) * (size_t)c->tslot * c->nslot) == cudaSuccess) {
-      if (cufftPlanMany(&c->yplan, 1, &ny, nullptr, 1, ny, nullptr, 1, ny, CUFFT_C2C, (int)yrows) == CUFFT_SUCCESS) {
-        c->allocs.push_back(tb);
-        c->tbuf = (float2 *)tb;
-        c->xtr = true;
-        c->yplan_ok = true;
-        CKFFT(c, cufftSetStream(c->yplan, c->stream));
-        c->plan_ok = true;  // the context is complete (c->plan is not used on this path)
-        return CAPOW_OK;
-      }
-      cudaFree(tb);
-    }
-    (void)cudaGetLastError();  // clear the failed allocation
-    c->fused = xbin_plan(bp, c->nslot, c->xg, false);
-  }
-  if (c->fused) {
-    int n2[2] = {p->NY, p->NZ};
-    int in2[2] = {p->NY, 2 * bp.nzc}, on2[2] = {p->NY, bp.nzc};
-    CKFFT(c, cufftPlanMany(&c->plan, 2, n2, in2, 1, p->NY * 2 * bp.nzc, on2, 1, p->NY * bp.nzc, CUFFT_R2C,
-                           p->NX * c->nslot));
-    c->plan_ok = true;
-    CKFFT(c, cufftSetStream(c->plan, c->stream));
-    return CAPOW_OK;
-  }
-  // one batched in-place r2c plan over all painted grids (replaces the fftw_execute calls,
-  // src/main.c:266-271): forward, unnormalised, padded last dimension
-  int n[3] = {p->NX, p->NY, p->NZ};
-  int inembed[3] = {p->NX, p->NY, 2 * bp.nzc}, onembed[3] = {p->NX, p->NY, bp.nzc};
-  long long idist = (long long)c->grid_elems, odist = (long long)c->grid_elems / 2;
-  if (idist > 0x7fffffffLL) {
-    // cufftPlanMany takes int distances; large grids use one plan per grid instead
-    CKFFT(c, cufftPlan3d(&c->plan, p->NX, p->NY, p->NZ, f64 ? CUFFT_D2Z : CUFFT_R2C));
-  } else {
-    CKFFT(c, cufftPlanMany(&c->plan, 3, n, inembed, 1, (int)idist, onembed, 1, (int)odist,
-                           f64 ? CUFFT_D2Z : CUFFT_R2C, c->nslot));
-  }
-  c->plan_ok = true;
-  CKFFT(c, cufftSetStream(c->plan, c->stream));
-  return CAPOW_OK;
+  return choose_layout(c, !ctx_no_blocked);
 }
 
 // A context that paints only: the grids, counters and FP32 tile buffers of capow_create, without bin
@@ -441,7 +473,7 @@ static int stage_input(capow_ctx *c, const capow_particles *in, capow_particles 
       if (c->stage[set][k]) cudaFree(c->stage[set][k]);
       c->stage[set][k] = nullptr;
       c->stage_bytes[set][k] = 0;
-      CK(c, cudaMalloc(&c->stage[set][k], bytes));
+      CK(c, ctx_malloc(c, (void **)&c->stage[set][k], bytes));
       c->stage_bytes[set][k] = bytes;
     }
     if (!chunked) CK(c, cudaMemcpyAsync(c->stage[set][k], src[k], bytes, cudaMemcpyHostToDevice, c->stream));
@@ -491,8 +523,8 @@ static int ensure_records(capow_ctx *c, unsigned long long need, bool weights) {
   c->pb.recs = nullptr;
   c->pb.recw = nullptr;
   c->pb.capacity = 0;
-  CK(c, cudaMalloc(&c->pb.recs, sizeof(float4) * need));
-  if (weights) CK(c, cudaMalloc(&c->pb.recw, sizeof(float) * need));
+  CK(c, ctx_malloc(c, (void **)&c->pb.recs, sizeof(float4) * need));
+  if (weights) CK(c, ctx_malloc(c, (void **)&c->pb.recw, sizeof(float) * need));
   c->pb.capacity = need;
   return CAPOW_OK;
 }
@@ -509,7 +541,7 @@ static int ensure_buckets(capow_ctx *c, unsigned long long n, bool weights) {
   int rc = ensure_records(c, (unsigned long long)bucket_capacity(c, n) * c->tg.ntiles, weights);
   if (rc) return rc;
   const unsigned long long ocap = n / 4 + 65536;
-  if (!c->pb.ovf_count) CK(c, cudaMalloc(&c->pb.ovf_count, sizeof(unsigned)));
+  if (!c->pb.ovf_count) CK(c, ctx_malloc(c, (void **)&c->pb.ovf_count, sizeof(unsigned)));
   if (c->pb.ovf_cap < ocap || (weights && !c->pb.ovf_w)) {
     if (c->pb.ovf_recs) cudaFree(c->pb.ovf_recs);
     if (c->pb.ovf_w) cudaFree(c->pb.ovf_w);
@@ -518,9 +550,9 @@ static int ensure_buckets(capow_ctx *c, unsigned long long n, bool weights) {
     c->pb.ovf_w = nullptr;
     c->pb.ovf_tile = nullptr;
     c->pb.ovf_cap = 0;
-    CK(c, cudaMalloc(&c->pb.ovf_recs, sizeof(float4) * ocap));
-    CK(c, cudaMalloc(&c->pb.ovf_tile, sizeof(unsigned) * ocap));
-    if (weights) CK(c, cudaMalloc(&c->pb.ovf_w, sizeof(float) * ocap));
+    CK(c, ctx_malloc(c, (void **)&c->pb.ovf_recs, sizeof(float4) * ocap));
+    CK(c, ctx_malloc(c, (void **)&c->pb.ovf_tile, sizeof(unsigned) * ocap));
+    if (weights) CK(c, ctx_malloc(c, (void **)&c->pb.ovf_w, sizeof(float) * ocap));
     c->pb.ovf_cap = ocap;
   }
   return CAPOW_OK;
@@ -536,12 +568,12 @@ int enqueue_paint(capow_ctx *c, const capow_particles &d) {
     CK(c, cudaMemsetAsync(c->grid_base, 0, 8 * c->grid_elems * c->nslot, c->stream));
     launch_paint64(c->stream, c->g, c->fs, d.dtype, d.x, d.y, d.z, d.vlos, d.w, n, gp, c->st, &c->launches);
   } else {
-    if (!c->pb.edge_count) CK(c, cudaMalloc(&c->pb.edge_count, sizeof(unsigned)));
+    if (!c->pb.edge_count) CK(c, ctx_malloc(c, (void **)&c->pb.edge_count, sizeof(unsigned)));
     if (c->pb.edge_cap < (unsigned long long)n + 1) {  // every particle could sit on an edge
       if (c->pb.edge_list) cudaFree(c->pb.edge_list);
       c->pb.edge_list = nullptr;
       c->pb.edge_cap = 0;
-      CK(c, cudaMalloc(&c->pb.edge_list, sizeof(unsigned) * (n + 1)));
+      CK(c, ctx_malloc(c, (void **)&c->pb.edge_list, sizeof(unsigned) * (n + 1)));
       c->pb.edge_cap = n + 1;
     }
     c->pb.bucket_cap = 0;
@@ -580,12 +612,12 @@ int enqueue_paint(capow_ctx *c, const capow_particles &d) {
 // allocates nothing.
 int prepare_paint_buffers(capow_ctx *c, unsigned long long nmax, bool weights) {
   if (c->prec == CAPOW_FP64) return CAPOW_OK;
-  if (!c->pb.edge_count) CK(c, cudaMalloc(&c->pb.edge_count, sizeof(unsigned)));
+  if (!c->pb.edge_count) CK(c, ctx_malloc(c, (void **)&c->pb.edge_count, sizeof(unsigned)));
   if (c->pb.edge_cap < nmax + 1) {
     if (c->pb.edge_list) cudaFree(c->pb.edge_list);
     c->pb.edge_list = nullptr;
     c->pb.edge_cap = 0;
-    CK(c, cudaMalloc(&c->pb.edge_list, sizeof(unsigned) * (nmax + 1)));
+    CK(c, ctx_malloc(c, (void **)&c->pb.edge_list, sizeof(unsigned) * (nmax + 1)));
     c->pb.edge_cap = nmax + 1;
   }
   if (c->prec == CAPOW_FP32_MIXED && !c->two_pass) return ensure_buckets(c, nmax, weights);
@@ -960,6 +992,10 @@ extern "C" void capow_destroy(capow_ctx *c) {
   for (int k = 0; k < 5; k++)
     if (c->adj_stage[k]) cudaFree(c->adj_stage[k]);
   for (void *p : c->allocs) cudaFree(p);
+  if (c->blk) {
+    cudaFree(c->tbuf);
+    cudaFree(c->ubuf);
+  }
   for (int s = 0; s < 2; s++) {
     for (int k = 0; k < 5; k++)
       if (c->stage[s][k]) cudaFree(c->stage[s][k]);

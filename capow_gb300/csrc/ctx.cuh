@@ -133,6 +133,10 @@ int enqueue_paint(capow_ctx *c, const capow_particles &d);
 // Set by a thread around capow_create: its context takes no blocked path. (A batch's mocks share contexts, and one whose
 // bins the blocked x pass cannot hold may fit the transposed one's.)
 extern thread_local bool ctx_no_blocked;
+// Give the blocked layout's buffers back for the layout without it (false: none to give back), and cudaMalloc with that as
+// its second try.
+bool leave_blocked(capow_ctx *c);
+cudaError_t ctx_malloc(capow_ctx *c, void **q, size_t bytes);
 int enqueue_power_kernels(capow_ctx *c);
 // Size the FP32 record and edge buffers (and, unless two_pass, the one-pass buckets at bucket_factor and
 // their overflow list) for catalogues of up to nmax particles, so that a later enqueue_paint allocates nothing.

@@ -1002,6 +1002,80 @@ static T *sv_upload(capow_survey_ctx *c, const std::vector<T> &h) {
 // cell-corner offset from the observer along one axis, as the reference forms it (src/main.c:554)
 static double corner(int i, double d, double mn, double o) { return (double)i * d + mn - o; }
 
+// The transform layout of a context whose tables and grids stand, and its buffer and plans. blocked: the blocked layout may
+// be taken.
+static int sv_choose_layout(capow_survey_ctx *c, bool blocked) {
+  // FP32 with a power-of-two NZ: the transposed path (its z pass weights the painted grids as it reads
+  // them, so no weighted grid is written; the y axis is then a contiguous batched transform)
+  const capow_params *p = &c->p;
+  const BinParams &bp = c->bp;
+  const bool f64 = c->prec == CAPOW_FP64;
+  const size_t ge = (size_t)c->g.main_sz;
+  if (!f64 && c->bt.twz && zr2c_supported(bp)) {
+    if (blocked && xrow_survey_plan(bp, c->bt, c->nslot, c->xg)) {
+      void *ub = nullptr;
+      c->uslot = (long long)(bp.kzmax + 1) * p->NY * p->NX;
+      if (cudaMalloc(&ub, sizeof(float2) * (size_t)c->uslot * c->nslot) == cudaSuccess) {
+        c->ubuf = (float2 *)ub;
+        c->tr = c->blk = true;
+        return CAPOW_OK;
+      }
+      (void)cudaGetLastError();  // no room: the transforms in place below
+    }
+    const long long yrows = (long long)c->nslot * p->NX * bp.nzc, xcols = (long long)bp.nzc * p->NY;
+    int ny = p->NY, nx = p->NX, emb = p->NX;
+    if (yrows <= 0x7fffffffLL && xcols <= 0x7fffffffLL &&
+        cufftPlanMany(&c->yplan, 1, &ny, nullptr, 1, ny, nullptr, 1, ny, CUFFT_C2C, (int)yrows) == CUFFT_SUCCESS) {
+      c->yplan_ok = true;
+      if (cufftPlanMany(&c->xplan, 1, &nx, &emb, (int)xcols, 1, &emb, (int)xcols, 1, CUFFT_C2C, (int)xcols) ==
+          CUFFT_SUCCESS) {
+        c->xplan_ok = true;
+        c->tr = true;
+        CKFFT(c, cufftSetStream(c->yplan, c->stream));
+        CKFFT(c, cufftSetStream(c->xplan, c->stream));
+        return CAPOW_OK;
+      }
+    }
+    (void)cudaGetLastError();  // no room for the plans: the 3-D transform below
+  }
+  // one batched in-place real-to-complex plan over the nslot term grids (fftw_execute of plan, plan_interlace,
+  // plan_mom and plan_mom_interlace, src/main.c:513-526 and the product loops)
+  int n[3] = {p->NX, p->NY, p->NZ};
+  int inembed[3] = {p->NX, p->NY, 2 * bp.nzc}, onembed[3] = {p->NX, p->NY, bp.nzc};
+  const long long idist = (long long)ge, odist = (long long)ge / 2;
+  if (idist > 0x7fffffffLL || c->nslot == 1) {
+    CKFFT(c, cufftPlan3d(&c->plan, p->NX, p->NY, p->NZ, f64 ? CUFFT_D2Z : CUFFT_R2C));
+    c->plan_per_grid = true;
+  } else {
+    CKFFT(c, cufftPlanMany(&c->plan, 3, n, inembed, 1, (int)idist, onembed, 1, (int)odist, f64 ? CUFFT_D2Z : CUFFT_R2C,
+                           c->nslot));
+  }
+  c->plan_ok = true;
+  CKFFT(c, cufftSetStream(c->plan, c->stream));
+  return CAPOW_OK;
+}
+
+// The blocked layout's buffer is memory that the other layouts do not take: when a later allocation finds no room, the context
+// gives it back and takes the layout that it would have had without it. False: it has none to give back.
+static bool sv_leave_blocked(capow_survey_ctx *c) {
+  if (!c->blk) return false;
+  (void)cudaGetLastError();
+  cudaStreamSynchronize(c->stream);
+  cudaFree(c->ubuf);
+  c->ubuf = nullptr;
+  c->tr = c->blk = false;
+  const int rc = sv_choose_layout(c, false);
+  (void)cudaGetLastError();
+  return rc == CAPOW_OK;
+}
+
+// cudaMalloc of a buffer that a context needs after its creation.
+static cudaError_t sv_malloc(capow_survey_ctx *c, void **q, size_t bytes) {
+  cudaError_t e = cudaMalloc(q, bytes);
+  if (e == cudaErrorMemoryAllocation && sv_leave_blocked(c)) e = cudaMalloc(q, bytes);
+  return e;
+}
+
 extern "C" int capow_survey_create(const capow_params *p, const capow_survey_params *sv, const capow_options *opt,
                                    capow_survey_ctx **out) {
   if (!p || !out) return CAPOW_EINVAL;
@@ -1137,51 +1211,7 @@ extern "C" int capow_survey_create(const capow_params *p, const capow_survey_par
   CK(c, cudaMemcpyAsync(c->nmodes.data(), c->nmodes_d, sizeof(unsigned long long) * nk, cudaMemcpyDeviceToHost,
                         c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
-  // FP32 with a power-of-two NZ: the transposed path (its z pass weights the painted grids as it reads
-  // them, so no weighted grid is written; the y axis is then a contiguous batched transform)
-  if (!f64 && c->bt.twz && zr2c_supported(bp)) {
-    if (xrow_survey_plan(bp, c->bt, c->nslot, c->xg)) {
-      void *ub = nullptr;
-      c->uslot = (long long)(bp.kzmax + 1) * p->NY * p->NX;
-      if (cudaMalloc(&ub, sizeof(float2) * (size_t)c->uslot * c->nslot) == cudaSuccess) {
-        c->allocs.push_back(ub);
-        c->ubuf = (float2 *)ub;
-        c->tr = c->blk = true;
-        return CAPOW_OK;
-      }
-      (void)cudaGetLastError();  // no room: the transforms in place below
-    }
-    const long long yrows = (long long)c->nslot * p->NX * bp.nzc, xcols = (long long)bp.nzc * p->NY;
-    int ny = p->NY, nx = p->NX, emb = p->NX;
-    if (yrows <= 0x7fffffffLL && xcols <= 0x7fffffffLL &&
-        cufftPlanMany(&c->yplan, 1, &ny, nullptr, 1, ny, nullptr, 1, ny, CUFFT_C2C, (int)yrows) == CUFFT_SUCCESS) {
-      c->yplan_ok = true;
-      if (cufftPlanMany(&c->xplan, 1, &nx, &emb, (int)xcols, 1, &emb, (int)xcols, 1, CUFFT_C2C, (int)xcols) ==
-          CUFFT_SUCCESS) {
-        c->xplan_ok = true;
-        c->tr = true;
-        CKFFT(c, cufftSetStream(c->yplan, c->stream));
-        CKFFT(c, cufftSetStream(c->xplan, c->stream));
-        return CAPOW_OK;
-      }
-    }
-    (void)cudaGetLastError();  // no room for the plans: the 3-D transform below
-  }
-  // one batched in-place real-to-complex plan over the nslot term grids (fftw_execute of plan, plan_interlace,
-  // plan_mom and plan_mom_interlace, src/main.c:513-526 and the product loops)
-  int n[3] = {p->NX, p->NY, p->NZ};
-  int inembed[3] = {p->NX, p->NY, 2 * bp.nzc}, onembed[3] = {p->NX, p->NY, bp.nzc};
-  const long long idist = (long long)ge, odist = (long long)ge / 2;
-  if (idist > 0x7fffffffLL || c->nslot == 1) {
-    CKFFT(c, cufftPlan3d(&c->plan, p->NX, p->NY, p->NZ, f64 ? CUFFT_D2Z : CUFFT_R2C));
-    c->plan_per_grid = true;
-  } else {
-    CKFFT(c, cufftPlanMany(&c->plan, 3, n, inembed, 1, (int)idist, onembed, 1, (int)odist, f64 ? CUFFT_D2Z : CUFFT_R2C,
-                           c->nslot));
-  }
-  c->plan_ok = true;
-  CKFFT(c, cufftSetStream(c->plan, c->stream));
-  return CAPOW_OK;
+  return sv_choose_layout(c, true);
 }
 
 extern "C" void capow_survey_destroy(capow_survey_ctx *c) {
@@ -1193,6 +1223,7 @@ extern "C" void capow_survey_destroy(capow_survey_ctx *c) {
   if (c->pc) capow_destroy(c->pc);
   if (c->comb) cudaFree(c->comb);
   for (void *q : c->allocs) cudaFree(q);
+  if (c->ubuf) cudaFree(c->ubuf);
   for (int a = 0; a < 2; a++)
     for (int k = 0; k < SV_STAGE; k++)
       if (c->stage[a][k]) cudaFree(c->stage[a][k]);
@@ -1213,7 +1244,7 @@ static int sv_stage_buffer(capow_survey_ctx *c, int cat, int k, size_t bytes) {
   if (c->stage[cat][k]) cudaFree(c->stage[cat][k]);
   c->stage[cat][k] = nullptr;
   c->stage_bytes[cat][k] = 0;
-  CK(c, cudaMalloc(&c->stage[cat][k], bytes ? bytes : 16));
+  CK(c, sv_malloc(c, &c->stage[cat][k], bytes ? bytes : 16));
   c->stage_bytes[cat][k] = bytes;
   return CAPOW_OK;
 }
@@ -1314,7 +1345,7 @@ static int sv_paint_tiles(capow_survey_ctx *c, const capow_survey_catalogue *dat
     if (c->comb) cudaFree(c->comb);
     c->comb = nullptr;
     c->comb_cap = 0;
-    CK(c, cudaMalloc(&c->comb, sizeof(float) * 5 * (n ? n : 1)));
+    CK(c, sv_malloc(c, (void **)&c->comb, sizeof(float) * 5 * (n ? n : 1)));
     c->comb_cap = n ? n : 1;
   }
   float *cx = c->comb, *cy = cx + c->comb_cap, *cz = cy + c->comb_cap, *cw = cz + c->comb_cap, *cv = cw + c->comb_cap;
@@ -1392,6 +1423,10 @@ static int sv_paint_tiles(capow_survey_ctx *c, const capow_survey_catalogue *dat
   const long long before = pc->launches;
   int rc = enqueue_paint(pc, d);
   if (!rc) rc = settle_paint(pc);
+  if (rc && cudaPeekAtLastError() == cudaErrorMemoryAllocation && sv_leave_blocked(c)) {  // no room for its records
+    rc = enqueue_paint(pc, d);
+    if (!rc) rc = settle_paint(pc);
+  }
   c->launches += pc->launches - before;
   if (rc) FAIL(c, rc, "survey paint: %s", capow_last_error(pc));
   return CAPOW_OK;

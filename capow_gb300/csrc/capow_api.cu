@@ -536,10 +536,26 @@ static unsigned bucket_capacity(const capow_ctx *c, unsigned long long n) {
   return ((unsigned)(f * mean) + 64 + 31) & ~31u;
 }
 
+// The smaller tiles of a small grid (fit_tiles) list a particle up to 1.7 times as often as the default ones. A catalogue whose
+// records find no room that way, or would leave 32 bits, takes the default tiles from then on (fewer of them: the tile tables
+// hold them). False: the context has them already.
+static bool take_default_tiles(capow_ctx *c) {
+  const TileGeo t = choose_tiles(c->g, c->nslot, c->prec == CAPOW_FP32_DETERMINISTIC);
+  if (t.ntiles >= c->tg.ntiles) return false;
+  (void)cudaGetLastError();
+  if (c->pb.recs) cudaFree(c->pb.recs);
+  if (c->pb.recw) cudaFree(c->pb.recw);
+  c->pb.recs = nullptr;
+  c->pb.recw = nullptr;
+  c->pb.capacity = 0;
+  c->tg = t;
+  return true;
+}
+
 // The bucket records and the overflow list of a one-pass paint of up to n particles.
 static int ensure_buckets(capow_ctx *c, unsigned long long n, bool weights) {
   int rc = ensure_records(c, (unsigned long long)bucket_capacity(c, n) * c->tg.ntiles, weights);
-  if (rc) return rc;
+  if (rc) return take_default_tiles(c) ? ensure_buckets(c, n, weights) : rc;
   const unsigned long long ocap = n / 4 + 65536;
   if (!c->pb.ovf_count) CK(c, ctx_malloc(c, (void **)&c->pb.ovf_count, sizeof(unsigned)));
   if (c->pb.ovf_cap < ocap || (weights && !c->pb.ovf_w)) {
@@ -550,14 +566,15 @@ static int ensure_buckets(capow_ctx *c, unsigned long long n, bool weights) {
     c->pb.ovf_w = nullptr;
     c->pb.ovf_tile = nullptr;
     c->pb.ovf_cap = 0;
-    CK(c, ctx_malloc(c, (void **)&c->pb.ovf_recs, sizeof(float4) * ocap));
-    CK(c, ctx_malloc(c, (void **)&c->pb.ovf_tile, sizeof(unsigned) * ocap));
-    if (weights) CK(c, ctx_malloc(c, (void **)&c->pb.ovf_w, sizeof(float) * ocap));
+    cudaError_t e = ctx_malloc(c, (void **)&c->pb.ovf_recs, sizeof(float4) * ocap);
+    if (e == cudaSuccess) e = ctx_malloc(c, (void **)&c->pb.ovf_tile, sizeof(unsigned) * ocap);
+    if (e == cudaSuccess && weights) e = ctx_malloc(c, (void **)&c->pb.ovf_w, sizeof(float) * ocap);
+    if (e == cudaErrorMemoryAllocation && take_default_tiles(c)) return ensure_buckets(c, n, weights);
+    CK(c, e);
     c->pb.ovf_cap = ocap;
   }
   return CAPOW_OK;
 }
-
 
 int enqueue_paint(capow_ctx *c, const capow_particles &d) {
   const long long n = (long long)d.n;
@@ -577,6 +594,7 @@ int enqueue_paint(capow_ctx *c, const capow_particles &d) {
       c->pb.edge_cap = n + 1;
     }
     c->pb.bucket_cap = 0;
+    if (tile_dup_estimate(c->g, c->tg) * (double)n > 4e9) take_default_tiles(c);
     if (c->prec == CAPOW_FP32_MIXED && !c->two_pass) {
       // bucket mode: each tile gets bucket_factor times its mean share of the records (plus slack); the
       // overflow list takes up to a quarter of the catalogue; beyond that the paint falls back to two passes
@@ -669,14 +687,14 @@ int settle_paint(capow_ctx *c) {
     CK(c, cudaMemcpyAsync(c->h_st, c->st, sizeof(DevStats), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
   }
-  if (c->h_st->overflow) {
+  for (int tries = 0; c->h_st->overflow; tries++) {
+    if (tries == 2) FAIL(c, CAPOW_ENOMEM, "tile record buffer overflow after resize");
     int rc = ensure_records(c, (unsigned long long)c->h_st->nrecords + 65536, c->last.w != nullptr);
-    if (rc) return rc;
+    if (rc && !take_default_tiles(c)) return rc;
     rc = enqueue_paint(c, c->last);
     if (rc) return rc;
     CK(c, cudaMemcpyAsync(c->h_st, c->st, sizeof(DevStats), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    if (c->h_st->overflow) FAIL(c, CAPOW_ENOMEM, "tile record buffer overflow after resize");
   }
   if (c->h_st->nonfinite) FAIL(c, CAPOW_EINVAL, "non-finite particle coordinate, velocity or weight");
   if (c->h_st->fatal) FAIL(c, CAPOW_EBOUNDS, "particle out of grid bounds with LOS == 0");
@@ -835,7 +853,7 @@ extern "C" int capow_power_result(capow_ctx *c, capow_spectrum *out, int nout) {
     int rc = CAPOW_OK;
     if (c->pb.bucket_cap) c->two_pass = true;  // the bucket overflow list filled
     else rc = ensure_records(c, (unsigned long long)c->h_st->nrecords + 65536, c->pend_last.w != nullptr);
-    if (rc) return rc;
+    if (rc && !take_default_tiles(c)) return rc;
     rc = enqueue_paint(c, c->pend_last);
     if (rc) return rc;
     rc = enqueue_power(c);

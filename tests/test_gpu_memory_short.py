@@ -138,3 +138,22 @@ def test_survey_after_a_blocked_context(gpu):
     (c0, a), (c1, b) = both(run, GRID // 2)
     assert abs(c0 - c1) < GRID // 8  # the blocked path in both contexts
     same([b], [a])
+
+
+def test_records_of_small_tiles(gpu):
+    """A grid of few tiles takes smaller ones, which list a particle more often: where their records do not fit, the default
+    tiles are taken."""
+    parts = particles(gpu, 8000000)
+
+    def run(held):
+        with cg.PowerSpectrum(params(NX=32, NY=32, NZ=32, Maxk=0.09, NK=10), precision="fp32") as ps:
+            ps.paint(*parts)
+            r = ps.power()
+            ps.paint(*parts)
+            ps.stats()
+            held()
+            return r, ps.tile_kernel_ms()[1]
+
+    (a, small), (b, default) = both(run, 100 << 20)
+    assert default < 0.8 * small  # records listed
+    same(b, a)

@@ -230,9 +230,9 @@ void relocate_bin_tables(BinTables &t, const void *base) {
 
 // exact 2-D mu bin, src/main.c:357-367, 454-455
 __device__ __forceinline__ int exact_mubin(const BinParams &bp, const BinTables &t, int i, int j, int k, double s) {
-  double fk = __dmul_rn(bp.two_pi, __dsqrt_rn(s));
+  double fk = __dmul_rn(2.0 * M_PI, __dsqrt_rn(s));
   double f = bp.los == 1 ? t.fxd[i] : (bp.los == 2 ? t.fyd[j] : t.fzd[k]);
-  double mu = fk > 0 ? __ddiv_rn(__dmul_rn(bp.two_pi, f), fk) : 0.0;
+  double mu = fk > 0 ? __ddiv_rn(__dmul_rn(2.0 * M_PI, f), fk) : 0.0;
   int mb = (int)__dmul_rn(__ddiv_rn(__dadd_rn(mu, 1.0), 2.0), (double)(float)bp.nmu);
   if (mb >= bp.nmu) mb = bp.nmu - 1;
   return mb;

@@ -956,9 +956,10 @@ static void launch_bucket(cudaStream_t s, const Geom &g, const FieldSpec &fs, co
   if (tg.ntiles <= BK_DIRECT_TILES) {
     const size_t smem = bucket_smem(tg.ntiles);
     allow_smem(k_bucket_cta<T>, 8192);
-    // one resident wave (two CTAs per SM); a small catalogue takes fewer particles per chunk, to fill it
+    // one resident wave (two CTAs per SM); a small catalogue takes fewer particles per chunk, to fill it, but as many as leave
+    // no second chunk to some of the CTAs
     const long long wave = 152LL * 2 * BK_THREADS;
-    const int ppt = (int)std::min<long long>(BK_PPT, std::max<long long>(1, n / wave));
+    const int ppt = (int)std::min<long long>(BK_PPT, std::max<long long>(1, (n + wave - 1) / wave));
     const long long chunks = (n + BK_THREADS * ppt - 1) / (BK_THREADS * ppt);
     const int nb = (int)(chunks < 1 ? 1 : (chunks > 152 * 2 ? 152 * 2 : chunks));
     k_bucket_cta<T><<<nb, BK_THREADS, smem, s>>>(g, fs, tg, in, n, ibase, ppt, b.counts, out, b.edge_list, b.edge_count,
@@ -1368,11 +1369,12 @@ __device__ void tile_paint_dense(const Geom &g, const FieldSpec &fs, const TileG
 // is staged. The cells are converted back to FP32 when the tile is written; in a cluster each CTA writes its
 // share of the tile as the sum of every CTA's cells (through distributed shared memory). (NGRID of these
 // particles is counted by the bucketing or k_count.)
+// (Four CTAs per SM for one slot, whose cells are 40 KB: 62 registers instead of 79.)
 template <int K, int NF, bool IL, bool CL>
-__global__ void __launch_bounds__(256, 3) k_tile_rec(Geom g, FieldSpec fs, TileGeo tg, const unsigned *offsets,
-                                                     const unsigned *counts, unsigned cap, const float4 *recs,
-                                                     const float *recw, unsigned long long capacity, int split,
-                                                     unsigned dense, GridPtrs grids, DevStats *st) {
+__global__ void __launch_bounds__(256, NF * (IL ? 2 : 1) == 1 && !CL ? 4 : 3)
+    k_tile_rec(Geom g, FieldSpec fs, TileGeo tg, const unsigned *offsets, const unsigned *counts, unsigned cap,
+               const float4 *recs, const float *recw, unsigned long long capacity, int split, unsigned dense, GridPtrs grids,
+               DevStats *st) {
   extern __shared__ __align__(16) int smi[];
   constexpr int NS = IL ? 2 : 1, SL = NS * NF;
   TileAt at;
@@ -1999,8 +2001,10 @@ size_t tile_smem_bytes(const TileGeo &tg, int nslots, int deterministic) {
   return ((size_t)nslots * tg.slot * (deterministic ? 8 : 4) + 15) & ~(size_t)15;
 }
 
-// k_tile_rec's cells: every slot, or for a dense tile the two limbs of one slot.
-size_t rec_smem_bytes(const TileGeo &tg, int nslots) { return (size_t)(nslots < 2 ? 2 : nslots) * tg.slot * 4; }
+// k_tile_rec's cells: every slot, or (dense) where a tile may be dense the two limbs of one slot if they are more.
+size_t rec_smem_bytes(const TileGeo &tg, int nslots, bool dense) {
+  return (size_t)(dense && nslots < 2 ? 2 : nslots) * tg.slot * 4;
+}
 
 double tile_dup_estimate(const Geom &g, const TileGeo &tg) {
   // a footprint spans 4 (TSC, CIC) or 2 (NN) cells plus the margin; it crosses into the next tile
@@ -2020,12 +2024,15 @@ static int rec_split(const TileGeo &tg, double records) {
 template <int K, int NF, bool IL>
 static void launch_rec(cudaStream_t s, const Geom &g, const FieldSpec &fs, const TileGeo &tg, const PaintBufs &b,
                        bool weights, long long n, const GridPtrs &grids, DevStats *st) {
-  const size_t smem = rec_smem_bytes(tg, NF * (IL ? 2 : 1));
   const int split = rec_split(tg, tile_dup_estimate(g, tg) * (double)n);
   const float *recw = weights ? b.recw : nullptr;
   const TileGeo def = choose_tiles(g, NF * (IL ? 2 : 1), 0);
   const unsigned dense = (unsigned)((double)TILE_DENSE_RECORDS * std::min(1.0, (double)tg.tx * tg.ty * tg.tz /
                                                                                ((double)def.tx * def.ty * def.tz)));
+  // (buckets that end below the dense limit: no tile needs the limbs' second slot. One slot, 512x256x256, TSC, 0.24M
+  // particles: 58 -> 57 us with 40 instead of 80 KB a CTA, 52 with the fourth CTA per SM that this leaves room for)
+  const bool may_dense = b.bucket_cap == 0 || b.bucket_cap > dense;
+  const size_t smem = rec_smem_bytes(tg, NF * (IL ? 2 : 1), may_dense);
   if (split > 1) {
     allow_smem(k_tile_rec<K, NF, IL, true>, 4096);
     cudaLaunchAttribute at;

@@ -85,5 +85,5 @@ TileGeo choose_tiles(const Geom &g, int nslots, int deterministic);
 TileGeo fit_tiles(const Geom &g, int nslots);  // FP32: smaller tiles where the default ones would be few
 TileGeo make_tiles(const Geom &g, int tx, int ty, int tz);  // tx, ty, tz powers of two (>= 4)
 size_t tile_smem_bytes(const TileGeo &tg, int nslots, int deterministic);
-size_t rec_smem_bytes(const TileGeo &tg, int nslots);
+size_t rec_smem_bytes(const TileGeo &tg, int nslots, bool dense);
 double tile_dup_estimate(const Geom &g, const TileGeo &tg);

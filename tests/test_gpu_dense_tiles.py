@@ -71,3 +71,16 @@ def test_one_record_far_above_the_others(gpu, shape, n, lo, hi, order, il):
         light = b < 2.0 ** 20
         assert np.array_equal(a[light], b[light]), f"{name}: largest difference {np.abs(a - b)[light].max()}"
         assert np.abs(a / np.where(light, 1.0, b) - 1.0)[~light].max(initial=0.0) <= 2.0 ** -23, name
+
+
+@pytest.mark.parametrize("shape,n,order", [((16, 16, 16), 1200, 2), ((16, 16, 16), 1900, 2), ((16, 16, 16), 2600, 1),
+                                           ((16, 16, 16), 4000, 1), ((32, 32, 32), 14000, 2), ((64, 64, 64), 155648, 2),
+                                           ((64, 64, 64), 155649, 3), ((64, 64, 64), 467000, 1)])
+def test_one_slot_around_the_bucket_limits(gpu, shape, n, order):
+    """One slot with buckets that end below and above the dense limit, half of the catalogue in one tile (beyond its bucket);
+    catalogues of one and more particles a thread of the bucketing."""
+    pos, v, w = catalogue(shape, n, order, n)
+    half, _, _ = catalogue(shape, n, order, n + 1, (1, 1, 1), (7, 7, 7))
+    pos = [np.where(np.arange(n) % 2 == 0, h, p) if n < 20000 else p for h, p in zip(half, pos)]
+    for name, a, b in paint(shape, order, 0, 0, 0, pos, np.zeros(n), w):
+        assert np.array_equal(a, b), f"{name}: largest difference {np.abs(a - b).max()}"

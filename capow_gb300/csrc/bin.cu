@@ -1233,7 +1233,7 @@ struct ZrGeo {
 
 // Geometry of a z pass over nslot grids ([NX][NY][row] floats, slot stride in_slot) into the transposed
 // slots (slot stride out_slot complex); nyb is set by the launcher from its rows per CTA.
-static ZrGeo zr2c_geo(const BinParams &bp, int nslot, long long in_slot, int row, long long out_slot) {
+static ZrGeo zr_geo(const BinParams &bp, int nslot, long long in_slot, int row, long long out_slot) {
   ZrGeo zg;
   int lm = 0;
   while ((2 << lm) < bp.nz) lm++;  // M = NZ / 2 = 2^lm
@@ -1505,10 +1505,10 @@ static void launch_zfft_m(cudaStream_t s, const ZrGeo &zg, const BinTables &t, i
   }
 }
 
-static void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+static void launch_zfft_any(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                         long long in_slot, int row, float2 *out, long long out_slot, const ZrWeight &w,
                         long long *launches, int x0, int nx) {
-  ZrGeo zg = zr2c_geo(bp, nslot, in_slot, row, out_slot);
+  ZrGeo zg = zr_geo(bp, nslot, in_slot, row, out_slot);
   if (nx >= 0) {
     zg.nx = nx;
     in += (long long)x0 * zg.slice;
@@ -1525,16 +1525,16 @@ static void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t,
   (*launches)++;
 }
 
-void launch_zr2c(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                  long long in_slot, int row, float2 *out, long long out_slot, long long *launches, int x0, int nx) {
-  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{nullptr, nullptr, nullptr, 0, 0}, launches, x0,
+  launch_zfft_any(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{nullptr, nullptr, nullptr, 0, 0}, launches, x0,
               nx);
 }
 
-void launch_zr2c_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+void launch_zfft_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                           long long in_slot, int row, float2 *out, long long out_slot, const float *vx,
                           const float *vy, const float *vz, int l, int m, long long *launches) {
-  launch_zfft(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{vx, vy, vz, l, m}, launches, 0, -1);
+  launch_zfft_any(s, bp, t, nslot, in, in_slot, row, out, out_slot, ZrWeight{vx, vy, vz, l, m}, launches, 0, -1);
 }
 
 // ------------------------------------------------------------ z and y axes in one launch (FP32)
@@ -1877,12 +1877,12 @@ __global__ void __launch_bounds__(ZR_THREADS, 4) k_zy(ZyGeo yg, BinTables t, con
   }
 }
 
-bool zr2c_supported(const BinParams &bp) {
+bool zfft_supported(const BinParams &bp) {
   return bp.nz >= 32 && bp.nz <= 2048 && (bp.nz & (bp.nz - 1)) == 0;
 }
 
 bool zy_supported(const BinParams &bp, const BinTables &t) {
-  return zr2c_supported(bp) && t.twy && bp.ny >= 16 && bp.ny <= 2048 && (bp.ny & (bp.ny - 1)) == 0;
+  return zfft_supported(bp) && t.twy && bp.ny >= 16 && bp.ny <= 2048 && (bp.ny & (bp.ny - 1)) == 0;
 }
 
 size_t zy_counter_words(const BinParams &bp, int nslot) { return 2 + (size_t)nslot * bp.nx; }

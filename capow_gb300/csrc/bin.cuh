@@ -38,7 +38,7 @@ struct BinTables {
 // Geometry of the fused x-axis FFT + binning pass (k_xfft_bin): blocks of `ncol` columns of the
 // (y, z)-transformed grids, `kc` consecutive "inner" indices of one "outer" index in each of the
 // nslot grids. Layout [NX][outer][inner]: tr = 0, [NX][NY][NZ/2+1] (outer ky, inner kz, after the
-// cuFFT 2-D transform); tr = 1, [NX][NZ/2+1][NY] (outer kz, inner ky, after k_zr2c and the y pass); tr = 2,
+// cuFFT 2-D transform); tr = 1, [NX][NZ/2+1][NY] (outer kz, inner ky, after k_zfft and the y pass); tr = 2,
 // [NZ/2+1][NY][NX] (k_yfft and k_xrow_bin, xbin.cu).
 struct XbinGeo {
   int log2n, ncol, log2ncol, kc, log2kc, nkb, nblocks;
@@ -116,7 +116,7 @@ int bin_products(int nfields);
 // (y, z)-transformed grids, x in real space, in the layout xg.tr names.
 bool xbin_plan(const BinParams &bp, int nslot, XbinGeo &xg, bool transposed);
 // The z-axis pass of the transposed fused layout: true when NZ is a power of two in [32, 2048].
-bool zr2c_supported(const BinParams &bp);
+bool zfft_supported(const BinParams &bp);
 // The z pass and the y-axis C2C of the transposed layout in one launch (power-of-two NZ and NY, the
 // tables' twy present). ctr: 2 + nslot * NX device counters, cleared by the launcher; a wait that gave
 // up sets st->timeout. stall != 0 (tests of the timeout path only) makes every wait run out.
@@ -130,11 +130,11 @@ void launch_zy(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslo
 // stride in_slot floats), out of place into out (slot stride out_slot complex) as [NX][NZ/2+1][NY].
 // The same z pass with the survey estimator's cell weights h_lm(r^) applied to the input as it is read (vx,
 // vy, vz: the cell-corner offsets from the observer per axis).
-void launch_zr2c_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+void launch_zfft_weighted(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                           long long in_slot, int row, float2 *out, long long out_slot, const float *vx,
                           const float *vy, const float *vz, int l, int m, long long *launches);
 // (x0, nx: only those planes, out then starting at plane x0)
-void launch_zr2c(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
+void launch_zfft(cudaStream_t s, const BinParams &bp, const BinTables &t, int nslot, const float *in,
                  long long in_slot, int row, float2 *out, long long out_slot, long long *launches, int x0 = 0,
                  int nx = -1);
 void launch_xbin(cudaStream_t s, const BinParams &bp, const BinTables &t, const XbinGeo &xg, void *const slots[4],

@@ -176,7 +176,7 @@ static int choose_layout(capow_ctx *c, bool blocked) {
   const bool f64 = c->prec == CAPOW_FP64;
   const bool want_fused = !f64 && o.fft_path != CAPOW_FFT_3D && c->bt.twx;
   const long long yrows = (long long)c->nslot * p->NX * bp.nzc;
-  const bool tr = want_fused && c->bt.twz && zr2c_supported(bp) && yrows <= 0x7fffffffLL;
+  const bool tr = want_fused && c->bt.twz && zfft_supported(bp) && yrows <= 0x7fffffffLL;
   if (tr && blocked && o.fft_path == CAPOW_FFT_AUTO && xrow_plan(bp, c->bt, c->nslot, c->xg)) {
     // power-of-two NY too: the blocked path. Its z and y passes run on up to 4 GB of planes at a time, so that a
     // large grid needs no third grid-sized buffer. (Each pair of launches costs about 20 us of ramps: at 512^3, runs
@@ -754,7 +754,7 @@ int enqueue_power_kernels(capow_ctx *c) {
     if (c->blk) {
       for (int x0 = 0; x0 < c->p.NX; x0 += c->planes) {
         const int nx = std::min(c->planes, c->p.NX - x0);
-        launch_zr2c(c->stream, c->bp, c->bt, c->nslot, (const float *)c->grid_base, (long long)c->grid_elems, c->g.row,
+        launch_zfft(c->stream, c->bp, c->bt, c->nslot, (const float *)c->grid_base, (long long)c->grid_elems, c->g.row,
                     c->tbuf, c->tslot, &c->launches, x0, nx);
         launch_yfft(c->stream, c->bp, c->bt, c->nslot, x0, nx, c->tbuf, c->tslot, c->ubuf, c->uslot);
       }
@@ -765,7 +765,7 @@ int enqueue_power_kernels(capow_ctx *c) {
       CK(c, cudaGetLastError());
       for (int k = 0; k < 4; k++) slots[k] = k < c->nslot ? (void *)(c->tbuf + c->tslot * k) : nullptr;
     } else if (c->xtr) {
-      launch_zr2c(c->stream, c->bp, c->bt, c->nslot, (const float *)c->grid_base, (long long)c->grid_elems, c->g.row,
+      launch_zfft(c->stream, c->bp, c->bt, c->nslot, (const float *)c->grid_base, (long long)c->grid_elems, c->g.row,
                   c->tbuf, c->tslot, &c->launches);
       CKFFT(c, cufftExecC2C(c->yplan, (cufftComplex *)c->tbuf, (cufftComplex *)c->tbuf, CUFFT_FORWARD));
       for (int k = 0; k < 4; k++) slots[k] = k < c->nslot ? (void *)(c->tbuf + c->tslot * k) : nullptr;

@@ -1011,7 +1011,7 @@ static int sv_choose_layout(capow_survey_ctx *c, bool blocked) {
   const BinParams &bp = c->bp;
   const bool f64 = c->prec == CAPOW_FP64;
   const size_t ge = (size_t)c->g.main_sz;
-  if (!f64 && c->bt.twz && zr2c_supported(bp)) {
+  if (!f64 && c->bt.twz && zfft_supported(bp)) {
     if (blocked && xrow_survey_plan(bp, c->bt, c->nslot, c->xg)) {
       void *ub = nullptr;
       c->uslot = (long long)(bp.kzmax + 1) * p->NY * p->NX;
@@ -1503,10 +1503,10 @@ static int sv_multipoles(capow_survey_ctx *c) {
         if (c->tr) {  // weighted z pass into the transposed work slots, then y and x in place
           const long long tslot = ge / 2;
           if (l == 0)
-            launch_zr2c(c->stream, c->bp, c->bt, c->nslot, (const float *)a[0], ge, (int)g.row, (float2 *)w[0],
+            launch_zfft(c->stream, c->bp, c->bt, c->nslot, (const float *)a[0], ge, (int)g.row, (float2 *)w[0],
                         tslot, &c->launches);
           else
-            launch_zr2c_weighted(c->stream, c->bp, c->bt, c->nslot, (const float *)a[0], ge, (int)g.row,
+            launch_zfft_weighted(c->stream, c->bp, c->bt, c->nslot, (const float *)a[0], ge, (int)g.row,
                                  (float2 *)w[0], tslot, (const float *)c->vx, (const float *)c->vy,
                                  (const float *)c->vz, l, m, &c->launches);
           if (c->blk) {

@@ -229,10 +229,10 @@ void relocate_bin_tables(BinTables &t, const void *base) {
 // ---------------------------------------------------------------------------------- device side
 
 // exact 2-D mu bin, src/main.c:357-367, 454-455
-__device__ __forceinline__ int exact_mubin(const BinParams &bp, const BinTables &t, int i, int j, int k, double s) {
-  double fk = __dmul_rn(2.0 * M_PI, __dsqrt_rn(s));
+__device__ __forceinline__ int exact_mubin(const BinCore &bp, const BinTables &t, int i, int j, int k, double s) {
+  double fk = __dmul_rn(bp.two_pi, __dsqrt_rn(s));
   double f = bp.los == 1 ? t.fxd[i] : (bp.los == 2 ? t.fyd[j] : t.fzd[k]);
-  double mu = fk > 0 ? __ddiv_rn(__dmul_rn(2.0 * M_PI, f), fk) : 0.0;
+  double mu = fk > 0 ? __ddiv_rn(__dmul_rn(bp.two_pi, f), fk) : 0.0;
   int mb = (int)__dmul_rn(__ddiv_rn(__dadd_rn(mu, 1.0), 2.0), (double)(float)bp.nmu);
   if (mb >= bp.nmu) mb = bp.nmu - 1;
   return mb;
@@ -410,7 +410,7 @@ CAPOW_HD BinSmem bin_smem_layout(unsigned rsize, int np, int nk, int n2d_sm, int
 // ODD: also the odd multipoles (src/main.c:445-449). OUT2D: the (k, mu) histogram (:453-461).
 // All accumulator indexing is compile-time, so the per-thread sums live in registers.
 template <typename R, int NF, bool ODD, bool OUT2D>
-__global__ void __launch_bounds__(256) k_bin(BinParams bp, BinTables t, const typename CT<R>::C *gA,
+__global__ void __launch_bounds__(256) k_bin(BinCore bp, BinTables t, const typename CT<R>::C *gA,
                                              const typename CT<R>::C *gB, const typename CT<R>::C *gAi,
                                              const typename CT<R>::C *gBi, const double *dcv, double *bins,
                                              double *bins2d, int ichunk, int sm2d) {

@@ -46,26 +46,31 @@ struct XbinGeo {
   int nbc;  // copies of the CTA's bins in shared memory (warps spread over them), a power of two
 };
 
-struct BinParams {
+struct BinCore {
   int nx, ny, nz, nzc, xhalf;
   int nk, nmu, los, interlace, odd, out2d;
   int nspec, nfields;
   SpecDef spec[CAPOW_MAX_SPEC];
   int mean_sub_a;           // field A had the mean subtracted (DC correction)
   int pmask;                // products the spectra read (bit q: |A|^2, Re A*B, Im A*B, |B|^2)
+  double two_pi;
   float fx_step;            // x frequency spacing 1/((float)NX*dx) (src/main.c:329), for per-column x ranges
   // first guess of a mode's bin from FP32 s = |f|^2 for linear bins: (int)(sqrtf(s) * kscale + koff), i.e.
   // (2 pi |f| - Mink) / binwidth (src/main.c:369-373); lg = 1 (log bins) bisects instead. The guess only
   // starts the walk over the safe FP32 edges, so its rounding does not matter.
   float kscale, koff;
   int lg;
+};
+// (k_bin takes this part alone: from 129 bytes on the compiler keeps a kernel's by-value copy in another way, and k_bin with
+// 2-D bins took 260 instead of 248 us, 512x256x256. The other kernels take the whole, 136 bytes, and are up to a percent faster
+// so: a survey's sets on 512^3, 17.37 against 17.50 ms.)
+static_assert(sizeof(BinCore) <= 128, "BinCore");
+
+struct BinParams : BinCore {
   int kzmax;  // kz rows beyond this one lie above the top bin edge: no stage needs them
   float fy_step, fz_step;  // y and z frequency spacings
   float ftop2;             // |f|^2 of the top bin edge (to FP32)
 };
-// (One word more, and the compiler treats the kernels' by-value copies differently: k_bin with 2-D bins took 5% longer at
-// 136 bytes, 512x256x256: 260 against 248 us.)
-static_assert(sizeof(BinParams) <= 128, "BinParams");
 
 // bin in [-1, NK] of an exact s: E[b+1] <= s < E[b+2]
 __device__ __forceinline__ int exact_bin(const double *E, int nk, double s, int guess) {

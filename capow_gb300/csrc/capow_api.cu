@@ -349,6 +349,7 @@ extern "C" int capow_create(const capow_params *p, const capow_options *opt, cap
   bp.nx = p->NX; bp.ny = p->NY; bp.nz = p->NZ; bp.nzc = p->NZ / 2 + 1; bp.xhalf = p->NX / 2;
   bp.nk = nk; bp.nmu = p->NMU; bp.los = p->LOS; bp.interlace = p->DoInterlacing;
   bp.odd = p->Odd_Multipoles; bp.out2d = p->Output2D; bp.nfields = c->fs.nfields;
+  bp.two_pi = 2.0 * M_PI;
   bp.fx_step = (float)(1.0 / ((float)p->NX * c->g.dx));
   bin_params_kguess(bp, *p);
   if (build_bin_tables(*p, c->g, c->prec, c->bt, c->allocs, c->stream)) FAIL(c, CAPOW_ENOMEM, "bin tables");

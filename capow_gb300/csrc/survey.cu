@@ -1200,6 +1200,7 @@ extern "C" int capow_survey_create(const capow_params *p, const capow_survey_par
   bp.nx = p->NX; bp.ny = p->NY; bp.nz = p->NZ; bp.nzc = p->NZ / 2 + 1; bp.xhalf = p->NX / 2;
   bp.nk = nk; bp.nmu = p->NMU; bp.los = 3; bp.interlace = p->DoInterlacing;
   bp.odd = p->Odd_Multipoles; bp.out2d = 0; bp.nfields = 1;
+  bp.two_pi = 2.0 * M_PI;
   bp.fx_step = (float)(1.0 / ((float)p->NX * g.dx));
   bin_params_kguess(bp, *p);
   if (build_bin_tables(*p, g, c->prec, c->bt, c->allocs, c->stream)) FAIL(c, CAPOW_ENOMEM, "bin tables");

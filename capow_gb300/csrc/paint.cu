@@ -1015,13 +1015,13 @@ __device__ __forceinline__ void stage_axis64(const Geom &g, const AxisTaps &t, i
 // Compile-time-order FP32 taps of one axis (kind 0: x, 1: y or z).
 // Power-of-two scale 2^S for a tile's int32 fixed-point cells. A record's taps add at most |w v^e|
 // to one slot, so no cell of the slot exceeds the tile's sum of |w v^e| over its records; that sum
-// (FP32, raised by 0.1 % for its own rounding) times 2^S <= 2^30 keeps every partial sum, with the
-// half-unit rounding of each deposit (one per record and cell), inside int32.
+// (FP32, raised by 0.1 % for its own rounding) times 2^S < 2^31 keeps every partial sum inside int32: the 0.1 % are two
+// million units, the half-unit roundings of a tile's deposits (one per record and cell, at most TILE_DENSE_RECORDS) 8192.
 __device__ __forceinline__ int tile_scale_exp(float sum_abs) {
   const float bound = sum_abs * 1.001f;
   if (!(bound > 0.0f) || !isfinite(bound)) return 0;
   const int e = ilogbf(bound);  // bound < 2^(e+1)
-  const int S = 29 - e;
+  const int S = 30 - e;
   return S > 100 ? 100 : (S < -100 ? -100 : S);
 }
 
@@ -1468,12 +1468,12 @@ __global__ void __launch_bounds__(256, NF * (IL ? 2 : 1) == 1 && !CL ? 4 : 3)
     return;
   }
   // The scale is set by the sum (tile_scale_exp). When keeping every deposit below 2^22 costs
-  // it at most 2 bits (an ordinary tile: hundreds of comparable records), the tile takes that scale
+  // it at most 3 bits (an ordinary tile: hundreds of comparable records), the tile takes that scale
   // and the fast rounding; otherwise (few records, or one dominant record) it keeps the sum's scale
   // and rounds by conversion.
   const int SAs = tile_scale_exp(ta), SBs = tile_scale_exp(tb);
   const int SAf = min(SAs, tile_scale_max(xa)), SBf = min(SBs, tile_scale_max(xb));
-  const bool fast = (SAs - SAf <= 2) && (NF == 1 || SBs - SBf <= 2);
+  const bool fast = (SAs - SAf <= 3) && (NF == 1 || SBs - SBf <= 3);
   const int SA = fast ? SAf : SAs, SB = fast ? SBf : SBs;
   const float scA = ldexpf(1.0f, SA), scB = ldexpf(1.0f, SB);
   if (CL && threadIdx.x == 0) {

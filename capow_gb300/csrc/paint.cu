@@ -2013,22 +2013,39 @@ double tile_dup_estimate(const Geom &g, const TileGeo &tg) {
   return (1.0 + (span - 1.0) / tg.tx) * (1.0 + (span - 1.0) / tg.ty) * (1.0 + (span - 1.0) / tg.tz);
 }
 
-// CTAs per tile (a cluster, a power of two up to 8): a grid of few tiles takes clusters that fill the chip (three
-// CTAs per SM), but no more CTAs than there are blocks of 128 records in a tile.
-static int rec_split(const TileGeo &tg, double records) {
-  int s = 1;
-  while (s < 8 && 2 * s * tg.ntiles <= 152 * 3 * 2 && records / tg.ntiles >= 128.0 * 2 * s) s *= 2;
-  return s;
+// CTAs per tile, a power of two up to 8 (a cluster shares the tile's records): the one whose busiest SM is done first. A CTA
+// costs a fixed time (its cells cleared and written, in a cluster also its barriers and the reading of the others' cells) and
+// its share of the deposits; an SM works through its CTAs' deposits 1.9 and 2.4 times as fast with two and with three of them
+// as with one. The times (us, fitted to 1080 launches: NN to TSC, one to four slots, 64 to 512 tiles, 80 to 200,000 records a
+// tile) only rank the four; a cluster has to win by 4 %, one of eight by 15 %. 128^3, two slots, 60,000 to 600,000 CIC
+// particles: one CTA 17 to 29 us, two 31 to 44; 48^3, two slots, TSC, 600,000: 160 us by one, 107 by two, 113 by four; 32^3,
+// 200,000: 158, 88, 60 and 72 us by one to eight.
+static int rec_split(const TileGeo &tg, int K, int slots, double records, unsigned dense) {
+  const double r = records / tg.ntiles, kwords = (double)tg.tx * tg.ty * tg.tz * std::max(slots, 2) / 1024.0;
+  const double dep = 0.18e-3 * r * (22.0 + (r > dense ? 2.2 : 1.0) * K * K * K * slots);
+  const double bias[4] = {1.0, 1.04, 1.04, 1.15};
+  int best = 0;
+  double best_t = 0.0;
+  for (int k = 0; k < 4 && (k == 0 || tg.ntiles << k <= 152 * 6); k++) {
+    const double ctas = std::max(1.0, ceil((double)(tg.ntiles << k) / 152.0 - 0.1));  // of the busiest SM
+    const double fix = 1.4 + 0.07 * kwords + (k ? 1.25 + 0.09 * kwords : 0.0);
+    const double t = bias[k] * (8.0 + ctas * fix + ctas / (1 << k) * dep / (ctas <= 1.0 ? 1.0 : (ctas <= 2.0 ? 1.9 : 2.4)));
+    if (k == 0 || t < best_t) {
+      best = k;
+      best_t = t;
+    }
+  }
+  return 1 << best;
 }
 
 template <int K, int NF, bool IL>
 static void launch_rec(cudaStream_t s, const Geom &g, const FieldSpec &fs, const TileGeo &tg, const PaintBufs &b,
                        bool weights, long long n, const GridPtrs &grids, DevStats *st) {
-  const int split = rec_split(tg, tile_dup_estimate(g, tg) * (double)n);
   const float *recw = weights ? b.recw : nullptr;
   const TileGeo def = choose_tiles(g, NF * (IL ? 2 : 1), 0);
   const unsigned dense = (unsigned)((double)TILE_DENSE_RECORDS * std::min(1.0, (double)tg.tx * tg.ty * tg.tz /
                                                                                ((double)def.tx * def.ty * def.tz)));
+  const int split = rec_split(tg, K, NF * (IL ? 2 : 1), tile_dup_estimate(g, tg) * (double)n, dense);
   // (buckets that end below the dense limit: no tile needs the limbs' second slot. One slot, 512x256x256, TSC, 0.24M
   // particles: 58 -> 57 us with 40 instead of 80 KB a CTA, 52 with the fourth CTA per SM that this leaves room for)
   const bool may_dense = b.bucket_cap == 0 || b.bucket_cap > dense;

@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(BK_THREADS, 2)
         }
       }
       __syncwarp();  // srec and sw of the warp's particles are written
-      add_entries(ft, li);
+      if (g.order > 1) add_entries(ft, li);  // (NN: all of them below, and an entry of none for each would fill the list)
     }
     __syncthreads();
     // the few particles near a face of the grid (for NN: all), by the full rules, in dense warps

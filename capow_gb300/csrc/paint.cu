@@ -756,7 +756,7 @@ struct BucketOut {
 // they cost no idle lanes, and lanes with equal tiles share one reservation of bucket slots. What bounds both
 // variants below is instruction issue. They differ in how slots are reserved.
 //
-// k_bucket_cta, for up to BK_DIRECT_TILES tiles: a CTA ranks the entries of a chunk of BK_THREADS * ppt
+// k_bucket_cta, for up to BK_DIRECT_TILES tiles of 64 particles and more: a CTA ranks the entries of a chunk of BK_THREADS * ppt
 // particles by shared counters of every tile, reserves each touched tile's slots with one global atomic, then
 // writes the records. With few tiles and particles in random order the global atomics of the warps would meet
 // on the same addresses: 2,097,152 such particles took 337 us into the 256 tiles of a 128^3 grid when each run
@@ -880,7 +880,7 @@ __global__ void __launch_bounds__(BK_THREADS, 2)
   sum.finish(st, ovf_full);
 }
 
-// k_bucket_warp, for more tiles: the lanes of a warp with equal tiles share one global atomic, two groups of 32
+// k_bucket_warp, for more tiles or fewer particles: the lanes of a warp with equal tiles share one global atomic, two groups of 32
 // entries at a time so that their atomics are in flight together, and the next particles' loads run behind
 // them. (A CTA-wide ranking through a hash table of the touched tiles was slower: 550 against 500 us for 16.7M
 // particles in lattice order at 512^3.)
@@ -953,7 +953,10 @@ static void launch_bucket(cudaStream_t s, const Geom &g, const FieldSpec &fs, co
                           long long n, long long ibase, const PaintBufs &b, DevStats *st) {
   const BucketOut out{b.recs,     in.w ? b.recw : nullptr, b.bucket_cap, b.ovf_recs, in.w ? b.ovf_w : nullptr,
                       b.ovf_tile, b.ovf_count,             b.ovf_cap};
-  if (tg.ntiles <= BK_DIRECT_TILES) {
+  // (Below 64 particles a tile the CTA's passes over its counters cost more than the warps' atomics: 20,000 and 100,000
+  // particles on 256^3 and 300x200x250, before the tiles: 36 -> 31 and 48 -> 41 us; above 250 in random order the CTAs win,
+  // 1M on 128^3: 64 against 165 us.)
+  if (tg.ntiles <= BK_DIRECT_TILES && n >= 64LL * tg.ntiles) {
     const size_t smem = bucket_smem(tg.ntiles);
     allow_smem(k_bucket_cta<T>, 8192);
     // one resident wave (two CTAs per SM); a small catalogue takes fewer particles per chunk, to fill it, but as many as leave

@@ -68,7 +68,8 @@ struct PaintBufs {
   const cudaEvent_t *chunk_ev;
 };
 
-// Grids of up to this many tiles are bucketed by k_bucket_cta (16 KB of counters), larger ones by k_bucket_warp.
+// Grids of up to this many tiles are bucketed by k_bucket_cta (16 KB of counters), larger ones, and catalogues of few
+// particles a tile, by k_bucket_warp.
 constexpr int BK_DIRECT_TILES = 4096;
 
 // host launchers (paint.cu)

@@ -75,10 +75,11 @@ def test_one_record_far_above_the_others(gpu, shape, n, lo, hi, order, il):
 
 @pytest.mark.parametrize("shape,n,order", [((16, 16, 16), 1200, 2), ((16, 16, 16), 1900, 2), ((16, 16, 16), 2600, 1),
                                            ((16, 16, 16), 4000, 1), ((32, 32, 32), 14000, 2), ((64, 64, 64), 155648, 2),
-                                           ((64, 64, 64), 155649, 3), ((64, 64, 64), 467000, 1)])
+                                           ((64, 64, 64), 155649, 3), ((64, 64, 64), 467000, 1),
+                                           ((64, 64, 64), 16383, 1), ((64, 64, 64), 16383, 3), ((64, 64, 64), 16384, 2)])
 def test_one_slot_around_the_bucket_limits(gpu, shape, n, order):
     """One slot with buckets that end below and above the dense limit, half of the catalogue in one tile (beyond its bucket);
-    catalogues of one and more particles a thread of the bucketing."""
+    catalogues of one and more particles a thread of the bucketing, and at the line between its two forms."""
     pos, v, w = catalogue(shape, n, order, n)
     half, _, _ = catalogue(shape, n, order, n + 1, (1, 1, 1), (7, 7, 7))
     pos = [np.where(np.arange(n) % 2 == 0, h, p) if n < 20000 else p for h, p in zip(half, pos)]

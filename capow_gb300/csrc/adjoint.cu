@@ -27,9 +27,11 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "ctx.cuh"
+#include "launch.cuh"
 #include "paint_dev.cuh"
 
 template <typename R>
@@ -513,29 +515,127 @@ __device__ __forceinline__ bool adj_fill_taps(AxisTapsF &t, float *dw) {
   return on >= 0;
 }
 
-// The exact path of one particle, out of line: it is rare, and inlined its registers were the gather's.
-template <typename T>
-static __device__ __noinline__ void adj_exact32(const Geom &g, const FieldSpec &fs, const PIn<T> &in, long long p,
-                                                const AdjGrids<float> &gr, const AdjScalars &as, T *ox, T *oy, T *oz, T *ov,
-                                                T *ow) {
-  adj_particle_exact<T, float>(g, fs, in, p, gr.s, as, ox, oy, oz, ov, ow);
+// The particles that k_adj_readout32 listed, by the exact FP64 rules. Eight lanes share one: lanes 0 to 2 form an axis each,
+// then the lanes take its K^3 taps in turn and add their sums up. Long lists (and NN's, a few percent of the catalogue with one
+// tap each) go one particle to a thread, which keeps the FP64 pipe's lanes full.
+// What bounds it: the latency of a particle's chain, 20 us for TSC and 13 for CIC by eight lanes, 40 to 60 one to a thread; a
+// long list the FP64 work, 10 us (CIC 6) and 7 us (CIC 5) a thousand. The two meet at 9,000 (CIC 7,000) particles: a whole
+// gradient of 200,000 on 128^3, TSC, 8,000 listed: 348 us; 32,000: 588 by lanes, 511 by threads. With these particles in
+// the readout (one kept the other 31 lanes of its warp waiting, and its registers or, out of line, its calls cost the gather):
+// 374 and 542.
+constexpr unsigned ADJ_GROUP_MAX = 8192;  // longest list that eight lanes share
+
+struct AdjGroup {
+  double w[3][3], dw[3][3];
+  int idx[3][3];  // -1: off
+};
+
+template <int K, int NF, typename T>
+__global__ void __launch_bounds__(64) k_adj_exact32(Geom g, FieldSpec fs, PIn<T> in, const unsigned *list,
+                                                    const unsigned *count, AdjGrids<float> gr, AdjScalars hs,
+                                                    const double *gamma0, T *ox, T *oy, T *oz, T *ov, T *ow) {
+  const unsigned n = *count;
+  g.order = K;
+  g.survey = 0;
+  fs.nfields = NF;
+  if (K == 1 || n > ADJ_GROUP_MAX) {
+    if (blockIdx.x * blockDim.x >= n) return;
+    const AdjScalars as = adj_scalars(g, hs, gamma0);
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+      adj_particle_exact<T, float>(g, fs, in, list[k], gr.s, as, ox, oy, oz, ov, ow);
+    return;
+  }
+  if (blockIdx.x * (blockDim.x >> 3) >= n) return;
+  __shared__ AdjGroup s_grp[8];
+  AdjGroup &q = s_grp[threadIdx.x >> 3];
+  const int sub = threadIdx.x & 7;
+  const AdjScalars as = adj_scalars(g, hs, gamma0);
+  const unsigned ng = gridDim.x * (blockDim.x >> 3), k0 = blockIdx.x * (blockDim.x >> 3);
+  for (unsigned kb = k0; kb < n; kb += ng) {  // (uniform over the block: the groups of one warp meet in __syncwarp)
+    const unsigned k = kb + (threadIdx.x >> 3);
+    const bool on = k < n;
+    const long long p = list[on ? k : kb];
+    double c[3] = {(double)in.x[p], (double)in.y[p], (double)in.z[p]};
+    const double v = fs.need_v ? (double)in.v[p] : 0.0, w = in.w ? (double)in.w[p] : 1.0;
+    const bool read = isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2]) && isfinite(v) && isfinite(w);
+    if (g.los >= 1 && g.los <= 3) {
+      const double s = rsd_shift64(g, g.los == 1 ? c[0] : (g.los == 2 ? c[1] : c[2]), v);
+      if (g.los == 1) c[0] = s;
+      else if (g.los == 2) c[1] = s;
+      else c[2] = s;
+    }
+    const int ax = min(sub, 2);  // this lane's axis
+    const double pos = ax == 0 ? c[0] : (ax == 1 ? c[1] : c[2]), half = ax == 0 ? g.hx : (ax == 1 ? g.hy : g.hz),
+                 mn = ax == 0 ? g.xmin : (ax == 1 ? g.ymin : g.zmin), d = ax == 0 ? g.dx : (ax == 1 ? g.dy : g.dz);
+    double g0[2] = {0.0, 0.0}, gs[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    bool accepted = false;
+    const int nst = g.interlace ? 2 : 1;
+#pragma unroll 1
+    for (int st = 0; st < nst; st++) {
+      double u = st ? DADD(pos, half) : pos;
+      AxisTaps t;
+      const bool acc = exact_axis(g, ax, u, t);
+      if (K == 3 && ax == 0 && g.los == 0 && DSUB(u, mn) < d) u = DADD(u, g.lx);  // (the scale exact_axis used)
+      double dw[3];
+      adj_axis_deriv(K, DDIV(DSUB(u, mn), d), dw);
+      __syncwarp();  // the previous stencil's taps have been read
+      if (sub < 3)
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+          q.w[sub][j] = t.w[j];
+          q.dw[sub][j] = dw[j];
+          q.idx[sub][j] = t.on[j] ? t.idx[j] : -1;
+        }
+      const unsigned accs = __ballot_sync(0xffffffffu, acc) >> (threadIdx.x & 24);
+      __syncwarp();
+      if ((accs & 7u) != 7u) continue;  // an axis refuses the particle
+      if (st == 0) accepted = true;
+      for (int e = sub; e < K * K * K; e += 8) {
+        const int ic = e / (K * K), ib = e / K % K, ia = e % K;
+        const int ix = q.idx[0][ia], iy = q.idx[1][ib], iz = q.idx[2][ic];
+        if (ix < 0 || iy < 0 || iz < 0) continue;
+        const long long L = canon_index(g, ix, iy, iz);
+        if (L < 0) continue;
+        const double wx = q.w[0][ia], wy = q.w[1][ib], wz = q.w[2][ic], dx = q.dw[0][ia], dy = q.dw[1][ib], dz = q.dw[2][ic];
+#pragma unroll
+        for (int f = 0; f < NF; f++) {
+          const double G = (double)gr.s[st * NF + f][L];
+          g0[f] += G * wx * wy * wz;
+          gs[f][0] += G * dx * wy * wz;
+          gs[f][1] += G * wx * dy * wz;
+          gs[f][2] += G * wx * wy * dz;
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int f = 0; f < NF; f++) {
+        g0[f] += __shfl_xor_sync(0xffffffffu, g0[f], o);
+#pragma unroll
+        for (int j = 0; j < 3; j++) gs[f][j] += __shfl_xor_sync(0xffffffffu, gs[f][j], o);
+      }
+    if (sub == 0 && on) adj_store(g, fs, v, w, g0, gs, accepted, read, as, p, ox, oy, oz, ov, ow);
+  }
 }
 
 // Step 4 for FP32 contexts: particles away from every edge of the reference's rules gather their
 // taps with the FP32 rules of the paint (the same ones that deposited them) and form their gradient in
-// FP32; the others take the exact FP64 path.
-// What bounds it: issue (62%) and the L1 (57%): 16.7M particles, TSC, interlaced, 256^3: 0.88 ms, 1.59 with tests of every
-// tap, 64-bit index arithmetic and the exact path inlined (HBM alone: 0.2).
+// FP32; the others are listed for k_adj_exact32.
+// What bounds it: issue and the L1: 16.7M particles, TSC, interlaced, 256^3: 0.63 ms and 0.02 for the list; 0.89 with the
+// listed particles' rules called here and 16 CTAs per SM of 7 resident, 1.59 with them inlined, tests of every tap and
+// 64-bit index arithmetic (HBM alone: 0.2). NN, 8M: 0.14 + 0.06 ms, 1.87 with the call, 1.57 inlined.
 template <int K, int NF, typename T>
 __global__ void __launch_bounds__(128) k_adj_readout32(Geom g, FieldSpec fs, PIn<T> in, long long n,
                                                        AdjGrids<float> gr, AdjScalars hs, const double *gamma0,
-                                                       T *ox, T *oy, T *oz, T *ov, T *ow) {
+                                                       unsigned *list, unsigned *count, T *ox, T *oy, T *oz, T *ov, T *ow) {
   const AdjScalars as = adj_scalars(g, hs, gamma0);
   const AdjK32 k32 = adj_k32(g, as);
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
     const Prep pr = prep32(g, fs, in, p);
     if (!pr.fin || is_edge(g, pr.sx, pr.sy, pr.sz)) {
-      adj_exact32<T>(g, fs, in, p, gr, as, ox, oy, oz, ov, ow);
+      list[atomicAdd(count, 1u)] = (unsigned)p;
       continue;
     }
     float g0[NF], gs[NF][3];
@@ -658,8 +758,18 @@ static void adj_readout(capow_ctx *c, long long n, const AdjScalars &hs, const d
   AdjGrids<float> gr;
   for (int s = 0; s < 4; s++) gr.s[s] = s < c->nslot ? (const float *)((char *)c->grid_base + eb * c->grid_elems * s) : nullptr;
   const int K = c->p.InterpOrder;
-#define ADJ_RUN32(KK, NFF) \
-  k_adj_readout32<KK, NFF, T><<<nb, 128, 0, c->stream>>>(c->g, c->fs, in, n, gr, hs, gamma0, o[0], o[1], o[2], o[3], o[4])
+  unsigned *list = c->pb.edge_list, *count = c->pb.edge_count;  // (capow_backward: n + 1 entries; the paint is done with them)
+  cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream);
+  // one resident wave of the readout: of 16 CTAs per SM, 7 resident, the last wave was a quarter full
+#define ADJ_RUN32(KK, NFF)                                                                                                  \
+  do {                                                                                                                      \
+    const int nw = std::min(nb, resident_ctas((const void *)k_adj_readout32<KK, NFF, T>, 128, 0));                          \
+    k_adj_readout32<KK, NFF, T><<<nw, 128, 0, c->stream>>>(c->g, c->fs, in, n, gr, hs, gamma0, list, count, o[0], o[1],    \
+                                                           o[2], o[3], o[4]);                                              \
+    k_adj_exact32<KK, NFF, T><<<152 * 8, 64, 0, c->stream>>>(c->g, c->fs, in, list, count, gr, hs, gamma0, o[0], o[1],      \
+                                                             o[2], o[3], o[4]);                                            \
+    c->launches++;                                                                                                          \
+  } while (0)
   if (c->fs.nfields == 2) {
     if (K == 3) ADJ_RUN32(3, 2);
     else if (K == 2) ADJ_RUN32(2, 2);
@@ -729,6 +839,7 @@ extern "C" int capow_backward(capow_ctx *c, const double *const *dL_dP, const ca
   CK(c, cudaMemcpyAsync(coef_f, coef32.data(), sizeof(float) * ncoef, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaMemsetAsync(gamma0, 0, 2 * sizeof(double), c->stream));
   int rc = make_3d_plans(c);
+  if (!rc && c->prec != CAPOW_FP64) rc = ensure_edge_list(c, (unsigned long long)n);  // (a noalloc paint has its own)
   if (rc) return rc;
   // ---- the forward's grids (repainted unless the power stage left them in place), full 3-D transform
   rc = enqueue_backward_paint(c);

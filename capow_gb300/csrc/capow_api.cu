@@ -576,6 +576,19 @@ static int ensure_buckets(capow_ctx *c, unsigned long long n, bool weights) {
   return CAPOW_OK;
 }
 
+// The list of the particles that take the exact rules, for catalogues of n: every particle could sit on an edge.
+int ensure_edge_list(capow_ctx *c, unsigned long long n) {
+  if (!c->pb.edge_count) CK(c, ctx_malloc(c, (void **)&c->pb.edge_count, sizeof(unsigned)));
+  if (c->pb.edge_cap < n + 1) {
+    if (c->pb.edge_list) cudaFree(c->pb.edge_list);
+    c->pb.edge_list = nullptr;
+    c->pb.edge_cap = 0;
+    CK(c, ctx_malloc(c, (void **)&c->pb.edge_list, sizeof(unsigned) * (n + 1)));
+    c->pb.edge_cap = n + 1;
+  }
+  return CAPOW_OK;
+}
+
 int enqueue_paint(capow_ctx *c, const capow_particles &d) {
   const long long n = (long long)d.n;
   GridPtrs gp = grid_ptrs(c);
@@ -585,26 +598,20 @@ int enqueue_paint(capow_ctx *c, const capow_particles &d) {
     CK(c, cudaMemsetAsync(c->grid_base, 0, 8 * c->grid_elems * c->nslot, c->stream));
     launch_paint64(c->stream, c->g, c->fs, d.dtype, d.x, d.y, d.z, d.vlos, d.w, n, gp, c->st, &c->launches);
   } else {
-    if (!c->pb.edge_count) CK(c, ctx_malloc(c, (void **)&c->pb.edge_count, sizeof(unsigned)));
-    if (c->pb.edge_cap < (unsigned long long)n + 1) {  // every particle could sit on an edge
-      if (c->pb.edge_list) cudaFree(c->pb.edge_list);
-      c->pb.edge_list = nullptr;
-      c->pb.edge_cap = 0;
-      CK(c, ctx_malloc(c, (void **)&c->pb.edge_list, sizeof(unsigned) * (n + 1)));
-      c->pb.edge_cap = n + 1;
-    }
+    int rc = ensure_edge_list(c, (unsigned long long)n);
+    if (rc) return rc;
     c->pb.bucket_cap = 0;
     if (tile_dup_estimate(c->g, c->tg) * (double)n > 4e9) take_default_tiles(c);
     if (c->prec == CAPOW_FP32_MIXED && !c->two_pass) {
       // bucket mode: each tile gets bucket_factor times its mean share of the records (plus slack); the
       // overflow list takes up to a quarter of the catalogue; beyond that the paint falls back to two passes
-      int rc = ensure_buckets(c, (unsigned long long)n, d.w != nullptr);
+      rc = ensure_buckets(c, (unsigned long long)n, d.w != nullptr);
       if (rc) return rc;
       c->pb.bucket_cap = bucket_capacity(c, (unsigned long long)n);
     } else {
       unsigned long long want = (unsigned long long)(tile_dup_estimate(c->g, c->tg) * 1.25 * n) + 65536;
       if (c->pb.capacity < want / 2 || (d.w && !c->pb.recw)) {
-        int rc = ensure_records(c, want, d.w != nullptr);
+        rc = ensure_records(c, want, d.w != nullptr);
         if (rc) return rc;
       }
     }
@@ -630,14 +637,8 @@ int enqueue_paint(capow_ctx *c, const capow_particles &d) {
 // allocates nothing.
 int prepare_paint_buffers(capow_ctx *c, unsigned long long nmax, bool weights) {
   if (c->prec == CAPOW_FP64) return CAPOW_OK;
-  if (!c->pb.edge_count) CK(c, ctx_malloc(c, (void **)&c->pb.edge_count, sizeof(unsigned)));
-  if (c->pb.edge_cap < nmax + 1) {
-    if (c->pb.edge_list) cudaFree(c->pb.edge_list);
-    c->pb.edge_list = nullptr;
-    c->pb.edge_cap = 0;
-    CK(c, ctx_malloc(c, (void **)&c->pb.edge_list, sizeof(unsigned) * (nmax + 1)));
-    c->pb.edge_cap = nmax + 1;
-  }
+  int rc = ensure_edge_list(c, nmax);
+  if (rc) return rc;
   if (c->prec == CAPOW_FP32_MIXED && !c->two_pass) return ensure_buckets(c, nmax, weights);
   const unsigned long long want = (unsigned long long)(tile_dup_estimate(c->g, c->tg) * 1.25 * nmax) + 65536;
   return ensure_records(c, want, weights);

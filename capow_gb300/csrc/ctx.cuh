@@ -130,6 +130,7 @@ int create_paint_ctx(const capow_params *p, const capow_options *o, int survey, 
 // sync, read the paint counters into c->h_st, repaint c->last when the tile lists overflowed
 int settle_paint(capow_ctx *c);
 int enqueue_paint(capow_ctx *c, const capow_particles &d);
+int ensure_edge_list(capow_ctx *c, unsigned long long n);
 // Set by a thread around capow_create: its context takes no blocked path. (A batch's mocks share contexts, and one whose
 // bins the blocked x pass cannot hold may fit the transposed one's.)
 extern thread_local bool ctx_no_blocked;

@@ -960,9 +960,15 @@ static void launch_bucket(cudaStream_t s, const Geom &g, const FieldSpec &fs, co
     const size_t smem = bucket_smem(tg.ntiles);
     allow_smem(k_bucket_cta<T>, 8192);
     // one resident wave (two CTAs per SM); a small catalogue takes fewer particles per chunk, to fill it, but as many as leave
-    // no second chunk to some of the CTAs
+    // no second chunk to some of the CTAs. No more than the list has room for, though: the entries beyond it make a global
+    // atomic each (small tiles, a particle near a face one entry more). 21 x 21 x 33, CIC, 535,000 particles by chunks of 4 a
+    // thread 182 us a call, of 3 162; TSC, 2M: 692 by 4, 466 by 3. The line at 0.65 of another particle: 4 against 3 at 3.56
+    // is 271 to 256 us, at 3.71 (48^3) 244 to 242 for 2M and 144 to 150 for 535,000.
     const long long wave = 152LL * 2 * BK_THREADS;
-    const int ppt = (int)std::min<long long>(BK_PPT, std::max<long long>(1, (n + wave - 1) / wave));
+    const double entries = tile_dup_estimate(g, tg) +
+                           (g.order > 1 ? 1.0 - (1.0 - 3.5 / g.nx) * (1.0 - 3.5 / g.ny) * (1.0 - 3.5 / g.nz) : 0.0);
+    const int fits = std::max(1, (int)((double)BK_E / (BK_THREADS * entries) + 0.35));
+    const int ppt = (int)std::min<long long>(std::min(BK_PPT, fits), std::max<long long>(1, (n + wave - 1) / wave));
     const long long chunks = (n + BK_THREADS * ppt - 1) / (BK_THREADS * ppt);
     const int nb = (int)(chunks < 1 ? 1 : (chunks > 152 * 2 ? 152 * 2 : chunks));
     k_bucket_cta<T><<<nb, BK_THREADS, smem, s>>>(g, fs, tg, in, n, ibase, ppt, b.counts, out, b.edge_list, b.edge_count,
